@@ -250,6 +250,10 @@ kf_status kf_pipeline_create(const kf_pipeline_config* config, kf_pipeline** out
         require(entries <= (1ull << 32), "Sparse block capacity out of range");
         p.block_table.resize(entries);
         p.null_bricks.resize(blocks);
+        for (int l = 0; l < 2; ++l) {
+          p.null_cells[l].resize(static_cast<size_t>(null_cells_along((g.res_x + 7) / 8, l)) *
+                                 null_cells_along((g.res_y + 7) / 8, l) * null_cells_along((g.res_z + 7) / 8, l));
+        }
         p.slot_block.resize(p.sparse_capacity);
         p.allocated.resize(2);
       } else {
@@ -515,13 +519,14 @@ kf_status kf_pipeline_download_skip_structures(kf_pipeline* pipeline, uint8_t* b
     require(pipeline != nullptr && brick_class != nullptr && brick_radius != nullptr && records != nullptr,
             "kf_pipeline_download_skip_structures: null argument");
     Pipeline& p = pipeline->impl;
-    require(p.view.table == nullptr && p.brick_class.count != 0 && p.brick_radius.count != 0,
+    require(p.view.table == nullptr && p.brick_class.count != 0 && p.brick_code.count != 0,
             "kf_pipeline_download_skip_structures: no skip structures (sparse storage, or no integration yet)");
     require(bricks == static_cast<size_t>(p.view.bx) * p.view.by * p.view.bz && bricks == p.brick_class.count,
             "kf_pipeline_download_skip_structures: brick count mismatch");
     check(cudaStreamSynchronize(p.stream), "skip structures sync");
     check(cudaMemcpy(brick_class, p.brick_class.ptr, bricks, cudaMemcpyDeviceToHost), "brick class download");
-    check(cudaMemcpy(brick_radius, p.brick_radius.ptr, bricks, cudaMemcpyDeviceToHost), "brick radius download");
+    check(cudaMemcpy(brick_radius, p.brick_code.ptr, bricks, cudaMemcpyDeviceToHost), "brick radius download");
+    for (size_t b = 0; b < bricks; ++b) brick_radius[b] >>= 2;  // class | radius << 2
     check(cudaMemcpy(records, p.stencil_bits.ptr, bricks * 32u * sizeof(uint32_t), cudaMemcpyDeviceToHost),
           "stencil records download");
   });

@@ -553,12 +553,13 @@ constexpr uint32_t kBrickRadiusCap = 7;
 __global__ void brick_radius_kernel(const uint8_t* __restrict__ brick_class, const uint8_t* __restrict__ lower,
                                     uint8_t* __restrict__ out, uint32_t bx, uint32_t by, uint32_t bz, int axis,
                                     const IcpState* __restrict__ state) {
+  // the last pass writes the brick's code (class | radius << 2)
   if (state != nullptr && state->failed) return;  // no integration this frame: the classes stand
   const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= bx * by * bz) return;
   const uint32_t c = brick_class[b];
   if (c != 1u && c != 2u) {
-    out[b] = 0;
+    out[b] = static_cast<uint8_t>(axis == 2 ? c : 0u);
     return;
   }
   const uint32_t coord = axis == 0 ? b % bx : (axis == 1 ? (b / bx) % by : b / (bx * by));
@@ -583,7 +584,7 @@ __global__ void brick_radius_kernel(const uint8_t* __restrict__ brick_class, con
     run = run && !(m < k);
     if (run) r = k;
   }
-  out[b] = static_cast<uint8_t>(r);
+  out[b] = static_cast<uint8_t>(axis == 2 ? (c | (r << 2)) : r);
 }
 
 // ---- band integration (BandIntegrationSweep<kDevice>, tsdf_integration.cu:
@@ -766,7 +767,8 @@ __global__ void sparse_assign_kernel(const uint32_t* __restrict__ marked, const 
                                      uint32_t words, const unsigned long long* __restrict__ allocated,
                                      unsigned long long capacity, unsigned long long* __restrict__ table,
                                      uint32_t table_mask, uint32_t* __restrict__ slot_block, uint32_t* __restrict__ list,
-                                     unsigned* __restrict__ count, uint8_t* __restrict__ null_bricks, uint32_t bx,
+                                     unsigned* __restrict__ count, uint8_t* __restrict__ null_bricks,
+                                     uint8_t* __restrict__ null4, uint8_t* __restrict__ null16, uint32_t bx,
                                      uint32_t by, uint32_t bz, const IcpState* __restrict__ state) {
   if (state != nullptr && state->failed) return;
   const uint32_t w = blockIdx.x * blockDim.x + threadIdx.x;
@@ -796,7 +798,10 @@ __global__ void sparse_assign_kernel(const uint32_t* __restrict__ marked, const 
       for (int d = 0; d < 8; ++d) {
         const int nx = x - (d & 1), ny = y - ((d >> 1) & 1), nz = z - (d >> 2);
         if (nx >= 0 && ny >= 0 && nz >= 0) {
-          null_bricks[(static_cast<size_t>(nz) * by + static_cast<uint32_t>(ny)) * bx + static_cast<uint32_t>(nx)] = 0;
+          const uint32_t ux = static_cast<uint32_t>(nx), uy = static_cast<uint32_t>(ny), uz = static_cast<uint32_t>(nz);
+          null_bricks[(static_cast<size_t>(uz) * by + uy) * bx + ux] = 0;
+          null4[((uz >> 2) * (((by - 1u) >> 2) + 1u) + (uy >> 2)) * (((bx - 1u) >> 2) + 1u) + (ux >> 2)] = 0;
+          null16[((uz >> 4) * (((by - 1u) >> 4) + 1u) + (uy >> 4)) * (((bx - 1u) >> 4) + 1u) + (ux >> 4)] = 0;
         }
       }
     }
@@ -875,7 +880,7 @@ void prepare_blocks(Pipeline& p, uint32_t width, uint32_t height, cudaStream_t s
       p.voxel_bits.resize(static_cast<size_t>(blocks) * 32u);
       p.stencil_bits.resize(static_cast<size_t>(blocks) * 32u);
       p.brick_class.resize(blocks);
-      p.brick_radius.resize(blocks);
+      p.brick_code.resize(blocks);
       p.radius_scratch.resize(2 * static_cast<size_t>(blocks));
     } else {
       p.new_bits.resize(words);
@@ -910,13 +915,16 @@ void reset_blocks(Pipeline& p, cudaStream_t s) {
   check(cudaMemsetAsync(p.voxel_bits.ptr, 0, p.voxel_bits.bytes(), s), "skip bits reset");
   check(cudaMemsetAsync(p.stencil_bits.ptr, 0, p.stencil_bits.bytes(), s), "skip bits reset");
   check(cudaMemsetAsync(p.brick_class.ptr, 1, p.brick_class.bytes(), s), "skip bits reset");
-  check(cudaMemsetAsync(p.brick_radius.ptr, 0, p.brick_radius.bytes(), s), "skip bits reset");
+  check(cudaMemsetAsync(p.brick_code.ptr, 1, p.brick_code.bytes(), s), "skip bits reset");  // class 1, radius 0
 }
 
 void reset_sparse(Pipeline& p, cudaStream_t s) {
   if (p.block_table.count == 0) return;
   check(cudaMemsetAsync(p.block_table.ptr, 0xFF, p.block_table.bytes(), s), "block table reset");  // kEmptyEntry
   check(cudaMemsetAsync(p.null_bricks.ptr, 1, p.null_bricks.bytes(), s), "sparse null bricks reset");
+  for (const auto& cells : p.null_cells) {
+    check(cudaMemsetAsync(cells.ptr, 1, cells.bytes(), s), "sparse null cells reset");
+  }
   check(cudaMemsetAsync(p.allocated.ptr, 0, p.allocated.bytes(), s), "sparse counter reset");
 }
 
@@ -971,7 +979,7 @@ void launch_integrate(Pipeline& p, const float4* table, uint32_t width, uint32_t
       sparse_assign_kernel<<<ceil_div(words, 256), 256, 0, s>>>(
           p.band_bits.ptr, p.new_bits.ptr, p.word_prefix.ptr, p.cta_prefix.ptr, words, p.allocated.ptr,
           p.sparse_capacity, p.block_table.ptr, p.view.table_mask, p.slot_block.ptr, p.block_list.ptr,
-          p.block_count.ptr, p.null_bricks.ptr,
+          p.block_count.ptr, p.null_bricks.ptr, p.null_cells[0].ptr, p.null_cells[1].ptr,
           p.view.bx, p.view.by, p.view.bz, state);
       check(cudaGetLastError(), "sparse_assign_kernel launch");
     } else {
@@ -1025,14 +1033,14 @@ void launch_integrate(Pipeline& p, const float4* table, uint32_t width, uint32_t
       p.brick_class.ptr, p.brick_dirty.ptr, p.view.bx, p.view.by, p.view.bz, p.config.raycast.corner_policy == KF_CORNERS_REQUIRE_ALL,
       state);
   check(cudaGetLastError(), "stencil_bits_kernel launch");
-  const uint32_t bricks = static_cast<uint32_t>(p.brick_radius.count);
+  const uint32_t bricks = static_cast<uint32_t>(p.brick_code.count);
   uint8_t* run_x = p.radius_scratch.ptr;
   uint8_t* square_xy = p.radius_scratch.ptr + bricks;
   brick_radius_kernel<<<ceil_div(bricks, 256u), 256, 0, s>>>(p.brick_class.ptr, nullptr, run_x, p.view.bx, p.view.by,
                                                               p.view.bz, 0, state);
   brick_radius_kernel<<<ceil_div(bricks, 256u), 256, 0, s>>>(p.brick_class.ptr, run_x, square_xy, p.view.bx,
                                                               p.view.by, p.view.bz, 1, state);
-  brick_radius_kernel<<<ceil_div(bricks, 256u), 256, 0, s>>>(p.brick_class.ptr, square_xy, p.brick_radius.ptr,
+  brick_radius_kernel<<<ceil_div(bricks, 256u), 256, 0, s>>>(p.brick_class.ptr, square_xy, p.brick_code.ptr,
                                                               p.view.bx, p.view.by, p.view.bz, 2, state);
   check(cudaGetLastError(), "brick_radius_kernel launch");
 }

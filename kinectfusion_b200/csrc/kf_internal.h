@@ -297,11 +297,12 @@ struct Pipeline {
   // Per brick: 1 = every stencil based in the brick is nullopt, 2 = every
   // one is exactly 1.0 (all eight corners observed with tsdf exactly 1).
   DeviceArray<uint8_t> brick_class;
-  // Per brick of class 1 or 2: the radius (in bricks, up to 7) of the cube of
-  // bricks around it that all share its class, inside the brick grid, 0 for
-  // mixed bricks (brick_radius_kernel); the raycast crosses such a cube at
-  // once.  radius_scratch holds the passes' run and square radii.
-  DeviceArray<uint8_t> brick_radius;
+  // Per brick: its class | r << 2, where r is the radius (in bricks, up to 7)
+  // of the cube of bricks around it that all share its class 1 or 2, inside
+  // the brick grid, 0 for mixed bricks (brick_radius_kernel); the raycast
+  // crosses such a cube at once.  radius_scratch holds the passes' run and
+  // square radii.
+  DeviceArray<uint8_t> brick_code;
   DeviceArray<uint8_t> radius_scratch;
   DeviceArray<uint32_t> band_bits;       // band integration: blocks the bands cross
   // band-march raycast (BasicBandBitmap, occupancy.hpp:240-278): block bits
@@ -311,6 +312,9 @@ struct Pipeline {
   // sparse storage: per block b (x-major), 1 while the blocks b + {0,1}^3 are
   // all unallocated (every trilinear stencil based in b is then nullopt)
   DeviceArray<uint8_t> null_bricks;
+  // and per cell of 4^3 and of 16^3 blocks (x-major), 1 while every block of
+  // the cell is such a block: the raycast crosses the cell at once
+  DeviceArray<uint8_t> null_cells[2];
   // Sparse storage (BlockRep, block_rep.hpp:26-110): the voxel-block hash
   // (block -> slot, kf_common.cuh block_table_lookup) of 2^k >= 2 x capacity
   // entries, `sparse_capacity` slots in the pools.
@@ -393,6 +397,13 @@ struct Pipeline {
   Maps& maps_for(uint32_t w, uint32_t h);
   void clear_graphs();
 };
+
+// Null cells along one axis of `blocks` blocks: cells of 4 (level 0) or 16
+// (level 1) blocks.
+inline uint32_t null_cells_along(uint32_t blocks, int level) {
+  const uint32_t shift = level == 0 ? 2u : 4u;
+  return ((blocks - 1u) >> shift) + 1u;
+}
 
 // Integration pixel table: depth meters (NaN if unusable), lambda, fusion
 // weight and colour, one float4 per pixel.

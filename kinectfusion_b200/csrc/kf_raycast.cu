@@ -32,12 +32,22 @@
 namespace kf {
 namespace {
 
-// Rays left in a warp at or below which they march cooperatively, in renders
-// that start with lanes to spare (fewer rays than lanes per warp).  Where
-// every lane starts with a ray the rays march alone to the end: there the
-// cooperative rounds' extra shuffles cost more than their speculation saves
-// (640x480 render 0.405 -> 0.388 ms without them, maps identical).
+// Rays left in a warp at or below which they march cooperatively, as long as
+// each of them repeats its last step (runs of nullopt samples one voxel apart
+// along the border of the observed space, runs of free space).  Rays whose
+// steps change with every sample gain nothing from the speculation and march
+// alone: their cooperative rounds only cost the shuffles.
+// With this rule instead of "always, and never where every lane starts with a
+// ray": 640x480 0.220 -> 0.204 ms, 160x120 0.154 -> 0.110 ms, a tracked frame
+// 0.842 -> 0.797 ms (limits of 4 and 16 rays: 0.833 and 0.814 ms).
 constexpr int kCoopLanes = 8;
+
+// Decided samples a ray may take in one round before the round's gathers.
+// With a ray per lane, 4 share the other lanes' gathers (1, 2, 4, 8:
+// 1001x747 render 0.491, 0.479, 0.451, 0.455 ms); with few rays per warp a
+// ray that waits for another's run only loses time (160x120 0.107 ms at 1,
+// 0.115 ms at 4).
+constexpr int kRunFull = 4, kRunFew = 1;
 
 struct RaycastParams {
   float min_depth, max_depth, step_scale;
@@ -45,7 +55,7 @@ struct RaycastParams {
   int cell_normals;
   int seed_previous;
   uint32_t rays_per_warp;  // 32: one lane per ray, 2D CTA tile; 16 or 8: warp tiles below
-  int coop_rays;           // kCoopLanes, or 0 when rays_per_warp is 32
+  int run;                 // decided samples per round (kRunFull, kRunFew)
 };
 
 // Pixel tile of one warp that holds `rays` rays (lanes 0..rays-1; the other
@@ -136,16 +146,18 @@ __device__ __forceinline__ bool in_grid(const VolumeDev& v, f3 g) {
          g.y < static_cast<float>(v.ry) && g.z < static_cast<float>(v.rz);
 }
 
-// Class of a stencil from its record: 1 = exactly 1.0, 2 = nullopt, 0 = not
-// decided by the stencil bits, the corner weights may decide (every observed
-// corner is exactly 1), 3 = not decided, only the gather decides (an observed
-// corner holds another value).
-__device__ __forceinline__ int record_class(uint4 r, uint32_t bit) {
-  const uint32_t undecided = bit < 32u ? r.x >> bit : r.y >> (bit - 32u);
-  const uint32_t one = bit < 32u ? r.z >> bit : r.w >> (bit - 32u);
-  if (undecided & 1u) return (one & 1u) ? 0 : 3;
-  return (one & 1u) ? 1 : 2;
+// Class of the stencil at (x, y) of a brick layer from the layer's record:
+// 1 = exactly 1.0, 2 = nullopt, 0 = not decided by the stencil bits, the
+// corner weights may decide (every observed corner is exactly 1), 3 = not
+// decided, only the gather decides (an observed corner holds another value).
+__device__ __forceinline__ int record_class(uint4 r, uint32_t x, uint32_t y) {
+  const uint32_t bit = (y & 3u) * 8u + x;
+  const uint32_t undecided = ((y & 4u) != 0u ? r.y : r.x) >> bit, one = ((y & 4u) != 0u ? r.w : r.z) >> bit;
+  return (undecided & 1u) ? 3 - 3 * static_cast<int>(one & 1u) : 2 - static_cast<int>(one & 1u);
 }
+
+// The float of a whole number below 2^23.
+__device__ __forceinline__ float small_float(uint32_t n) { return __uint_as_float(0x4B000000u | n) - 8388608.0f; }
 
 // Ray parameter up to which the samples' stencil bases stay in a box of
 // bricks: the box of `size` voxels per axis whose lowest voxel is (lox, loy,
@@ -158,8 +170,8 @@ __device__ __forceinline__ int record_class(uint4 r, uint32_t bit) {
 __device__ __forceinline__ float box_exit(const VolumeDev& v, f3 g0, f3 inv_gdir, uint32_t lox, uint32_t loy,
                                           uint32_t loz, uint32_t size, bool clip, float margin) {
   auto axis = [margin, clip, size](float g, float inv, uint32_t lo_voxel, uint32_t extent) {
-    const float lo = static_cast<float>(lo_voxel) + 0.5f + margin;
-    float hi = static_cast<float>(lo_voxel + size) + 0.5f - margin;
+    const float lo = small_float(lo_voxel) + 0.5f + margin;
+    float hi = small_float(lo_voxel + size) + 0.5f - margin;
     if (clip) hi = fminf(hi, static_cast<float>(extent) - margin);
     return ((inv >= 0.0f ? hi : lo) - g) * inv;
   };
@@ -167,46 +179,45 @@ __device__ __forceinline__ float box_exit(const VolumeDev& v, f3 g0, f3 inv_gdir
                                                           axis(g0.z, inv_gdir.z, loz, v.rz)));
 }
 
-// A march sample: nullopt, a value, or past the march's end.
-enum : int { kNull = 0, kValue = 1, kEnd = 2 };
+// A march sample: nullopt or a value.
+enum : int { kNull = 0, kValue = 1 };
 // What a sample does to the march: nothing, a zero crossing, the end.
 enum : int { kNone = 0, kFound = 1, kStop = 2 };
 
-// The skip structures of a render: dense storage has the stencil records,
-// brick classes and cube radii (null before the first integration), sparse
-// storage the null-block flags.
+// The skip structures of a render: dense storage has the stencil records and
+// the brick codes (class | cube radius << 2; null before the first
+// integration), sparse storage the null-block flags and their coarse cells
+// of 4^3 and 16^3 blocks.
 struct SkipDev {
   const uint32_t* __restrict__ voxel_bits;
   const uint4* __restrict__ stencil_bits;
-  const uint8_t* __restrict__ brick_class;
-  const uint8_t* __restrict__ brick_radius;
+  const uint8_t* __restrict__ brick_code;
   const uint8_t* __restrict__ null_bricks;
+  const uint8_t* __restrict__ null_cells[2];
+  uint32_t cells_x[2], cells_y[2];
 };
 
-// A sample no stencil record settles: below the volume's first voxel centre
-// (no record there), or within a hair of a voxel plane (the weights of the
-// observed corners may fail the sampler's 1e-6 test).  Decided from the
+// A sample no stencil record settles: its stencil reaches outside the volume
+// (there are no records below the first voxel centre), it lies within a hair
+// of a voxel plane (the weights of the observed corners may fail the sampler's
+// 1e-6 test), or the volume has no skip structures yet.  Decided from the
 // per-voxel bits, else gathered.  Rare, and kept out of the march's code.
 template <int Kind>
 __device__ __noinline__ int rare_sample(const VolumeDev& v, const uint32_t* __restrict__ voxel_bits, int policy,
                                         f3 point, float& tsdf) {
   const f3 g = (point - v.origin) * v.inv_voxel_size;
-  uint32_t observed, one;
-  stencil_masks(voxel_bits, v, static_cast<int>(floorf(g.x - 0.5f)), static_cast<int>(floorf(g.y - 0.5f)),
-                static_cast<int>(floorf(g.z - 0.5f)), observed, one);
-  const int cls = stencil_class(observed, one, policy, g);
-  if (cls == 2) return kNull;
-  if (cls == 1) {
-    tsdf = 1.0f;
-    return kValue;
+  if (!in_grid(v, g)) return kNull;
+  if (voxel_bits != nullptr) {
+    uint32_t observed, one;
+    stencil_masks(voxel_bits, v, static_cast<int>(floorf(g.x - 0.5f)), static_cast<int>(floorf(g.y - 0.5f)),
+                  static_cast<int>(floorf(g.z - 0.5f)), observed, one);
+    const int cls = stencil_class(observed, one, policy, g);
+    if (cls == 2) return kNull;
+    if (cls == 1) {
+      tsdf = 1.0f;
+      return kValue;
+    }
   }
-  return Sampler<Kind>{v}.tsdf(point, policy, tsdf) ? kValue : kNull;
-}
-
-// Sampler::tsdf out of line, for samples whose stencil is clipped by the
-// volume's border or whose volume has no skip structures yet.
-template <int Kind>
-__device__ __noinline__ int clipped_sample(const VolumeDev& v, int policy, f3 point, float& tsdf) {
   return Sampler<Kind>{v}.tsdf(point, policy, tsdf) ? kValue : kNull;
 }
 
@@ -234,80 +245,97 @@ __device__ __forceinline__ int blend(const typename VoxelTraits<Kind>::Raw (&r)[
   return kValue;
 }
 
-// The sample at `point` (find_zero_crossing's volume.tsdf, raycasting.hpp:
-// 176-205): kNull or kValue with its value in `tsdf`.  With the skip
-// structures, a sample the stencil bits decide needs no corner gather, and
-// `jump` gets its brick (bit 31 | x | y << 10 | z << 20) when every stencil
-// of that brick has the sample's class, with `radius` the radius in bricks
-// of the cube around it whose bricks all have that class.
-//
-// A warp's lanes march different rays, so a round costs the sum of every
-// path some lane takes.  There is one path for nearly all samples: the
-// record, then (where it says so) one gather of the eight corners, whose
-// offsets step over brick borders instead of taking a second, clipped path.
-// With this and replay_steps a 640x480 render of a 512^3 volume went from
-// 0.440 to 0.308 ms and a tracked frame from 1.21 to 0.89 ms (both bound by
-// the rounds of the warps' longest rays and the instructions of a round).
-template <int Kind, bool Sparse>
-__device__ __forceinline__ int march_sample(const VolumeDev& v, const SkipDev& skip, int policy, f3 point, float& tsdf,
-                                            uint32_t& jump, uint32_t& radius) {
-  using VT = VoxelTraits<Kind>;
-  using Raw = typename VT::Raw;
-  jump = 0u;
-  radius = 0u;
+// What the skip structures say about a sample: its record's class
+// (record_class), where `weigh` stencils are already decided.
+enum : int { kRare = 0, kOne = 1, kNullopt = 2, kGather = 3 };
+
+// Where a sample's stencil sits: base voxel, brick and fractions; and for a
+// decided sample, the box of bricks it may cross because every stencil based
+// in it has the sample's class: `box` bricks on a side (0: none), the lowest
+// one packed as x | y << 10 | z << 20.
+struct Spot {
+  f3 fr;
+  uint32_t x, y, z, brick;
+  uint32_t box, lowest;
+};
+
+// The class of the sample at `point` from the skip structures alone: kOne
+// (exactly 1.0), kNullopt, kGather (the corners decide), kRare (rare_sample:
+// its stencil reaches outside the volume, among others).
+template <bool Sparse>
+__device__ __forceinline__ int decide(const VolumeDev& v, const SkipDev& skip, f3 point, Spot& at) {
+  at.box = 0u;
   const f3 g = (point - v.origin) * v.inv_voxel_size;
-  if (!in_grid(v, g)) return kNull;
   const f3 gg = make(g.x - 0.5f, g.y - 0.5f, g.z - 0.5f);
-  const f3 fl = make(floorf(gg.x), floorf(gg.y), floorf(gg.z));
-  const int sx = static_cast<int>(fl.x), sy = static_cast<int>(fl.y), sz = static_cast<int>(fl.z);
-  const uint32_t ux = static_cast<uint32_t>(sx), uy = static_cast<uint32_t>(sy), uz = static_cast<uint32_t>(sz);
-  const uint32_t bx = ux >> 3, by = uy >> 3, bz = uz >> 3;
-  const bool based = (sx | sy | sz) >= 0;
+  // floor by a round-down add of 2^23: the integer sits in the low mantissa
+  // bits; negative, huge and NaN positions give words past the extent
+  const f3 big = make(__fadd_rd(gg.x, 8388608.0f), __fadd_rd(gg.y, 8388608.0f), __fadd_rd(gg.z, 8388608.0f));
+  at.x = __float_as_uint(big.x) - 0x4B000000u;
+  at.y = __float_as_uint(big.y) - 0x4B000000u;
+  at.z = __float_as_uint(big.z) - 0x4B000000u;
+  // both corners of every axis inside the volume; so is the position then
+  if (at.x >= v.rx - 1u || at.y >= v.ry - 1u || at.z >= v.rz - 1u) return kRare;
+  at.fr = gg - make(big.x - 8388608.0f, big.y - 8388608.0f, big.z - 8388608.0f);
+  const uint32_t bx = at.x >> 3, by = at.y >> 3, bz = at.z >> 3;
+  at.brick = (bz * v.by + by) * v.bx + bx;
+  const bool packable = (bx | by | bz) < 1024u;
   if constexpr (Sparse) {
     // a stencil based in a block whose 2x2x2 block neighbourhood is
-    // unallocated has no observed corner
-    if (based && __ldg(skip.null_bricks + (static_cast<size_t>(bz) * v.by + by) * v.bx + bx)) {
-      if (bx < 1024u && by < 1024u && bz < 1024u) jump = 0x80000000u | bx | (by << 10) | (bz << 20);
-      return kNull;
+    // unallocated has no observed corner; neither has one based in a coarse
+    // cell of such blocks
+    const bool null1 = __ldg(skip.null_bricks + at.brick) != 0;
+    const bool null4 = __ldg(skip.null_cells[0] + (((bz >> 2) * skip.cells_y[0] + (by >> 2)) * skip.cells_x[0] + (bx >> 2))) != 0;
+    const bool null16 = __ldg(skip.null_cells[1] + (((bz >> 4) * skip.cells_y[1] + (by >> 4)) * skip.cells_x[1] + (bx >> 4))) != 0;
+    if (!null1) return kGather;
+    const uint32_t shift = null16 ? 4u : (null4 ? 2u : 0u);
+    if (packable) {
+      at.box = 1u << shift;
+      at.lowest = ((bx >> shift) | ((by >> shift) << 10) | ((bz >> shift) << 20)) << shift;
     }
-    return Sampler<Kind>{v}.tsdf(point, policy, tsdf) ? kValue : kNull;
+    return kNullopt;
   } else {
-    if (skip.stencil_bits == nullptr) return clipped_sample<Kind>(v, policy, point, tsdf);
-    if (!based) return rare_sample<Kind>(v, skip.voxel_bits, policy, point, tsdf);
-    const uint32_t brick = (bz * v.by + by) * v.bx + bx;
-    const uint4 rec = __ldg(skip.stencil_bits + (static_cast<size_t>(brick) * 8u + (uz & 7u)));
-    const int summary = __ldg(skip.brick_class + brick);
-    const uint32_t cube = __ldg(skip.brick_radius + brick);
-    const f3 fr = gg - fl;
-    int cls = record_class(rec, (uy & 7u) * 8u + (ux & 7u));
+    if (skip.stencil_bits == nullptr) return kRare;
+    const uint4 rec = __ldg(skip.stencil_bits + (static_cast<size_t>(at.brick) * 8u + (at.z & 7u)));
+    const uint32_t code = __ldg(skip.brick_code + at.brick);
+    int cls = record_class(rec, at.x & 7u, at.y & 7u);
     if (cls == 0) {
       // every observed corner is exactly 1: the value is 1.0 once their
       // weights pass the 1e-6 test, which one corner's weight alone does
       // unless the sample all but touches a voxel plane (float products and
       // sums of non-negative terms are monotonic)
-      const float least = fminf(fr.x, 1.0f - fr.x) * fminf(fr.y, 1.0f - fr.y) * fminf(fr.z, 1.0f - fr.z);
-      if (!(least > 1.0e-6f)) return rare_sample<Kind>(v, skip.voxel_bits, policy, point, tsdf);
-      cls = 1;
+      const float least = fminf(at.fr.x, 1.0f - at.fr.x) * fminf(at.fr.y, 1.0f - at.fr.y) *
+                          fminf(at.fr.z, 1.0f - at.fr.z);
+      if (!(least > 1.0e-6f)) return kRare;
+      return kOne;  // its brick is mixed
     }
-    if (cls != 3) {
-      if (summary == (cls == 1 ? 2 : 1) && bx < 1024u && by < 1024u && bz < 1024u) {
-        jump = 0x80000000u | bx | (by << 10) | (bz << 20);
-        radius = cube;
-      }
-      tsdf = 1.0f;
-      return cls == 1 ? kValue : kNull;
+    // a brick of one class (1 nullopt, 2 one) holds only stencils of it
+    if ((code & 3u) != 0u && packable) {
+      const uint32_t radius = code >> 2;
+      at.box = 2u * radius + 1u;
+      at.lowest = (bx - radius) | ((by - radius) << 10) | ((bz - radius) << 20);
     }
-    if (ux + 1u >= v.rx || uy + 1u >= v.ry || uz + 1u >= v.rz) return clipped_sample<Kind>(v, policy, point, tsdf);
-    const Raw* b = reinterpret_cast<const Raw*>(v.voxels) +
-                   (static_cast<size_t>(brick) * 512u + ((uz & 7u) * 64u + (uy & 7u) * 8u + (ux & 7u)));
-    const size_t ox = (ux & 7u) == 7u ? 512u - 7u : 1u;
-    const size_t oy = (uy & 7u) == 7u ? v.bx * 512u - 56u : 8u;
-    const size_t oz = (uz & 7u) == 7u ? static_cast<size_t>(v.bx * v.by) * 512u - 448u : 64u;
-    Raw r[8];
-#pragma unroll
-    for (int c = 0; c < 8; ++c) r[c] = __ldg(b + ((c & 1 ? ox : 0u) + (c & 2 ? oy : 0u) + (c & 4 ? oz : 0u)));
-    return blend<Kind>(r, fr, policy, tsdf);
+    return cls;
   }
+}
+
+// The value of a sample that `decide` left to the corners (kGather, kRare):
+// TrilinearSampler::tsdf.  One gather whose offsets step over brick borders
+// serves every stencil inside the volume.
+template <int Kind, bool Sparse>
+__device__ __forceinline__ int resolve(const VolumeDev& v, const SkipDev& skip, int policy, f3 point, int cls,
+                                       const Spot& at, float& tsdf) {
+  using Raw = typename VoxelTraits<Kind>::Raw;
+  if (cls == kRare) return rare_sample<Kind>(v, skip.voxel_bits, policy, point, tsdf);
+  if constexpr (Sparse) return Sampler<Kind>{v}.tsdf(point, policy, tsdf) ? kValue : kNull;
+  const Raw* b = reinterpret_cast<const Raw*>(v.voxels) +
+                 (static_cast<size_t>(at.brick) * 512u + ((at.z & 7u) * 64u + (at.y & 7u) * 8u + (at.x & 7u)));
+  const size_t ox = (at.x & 7u) == 7u ? 512u - 7u : 1u;
+  const size_t oy = (at.y & 7u) == 7u ? v.bx * 512u - 56u : 8u;
+  const size_t oz = (at.z & 7u) == 7u ? static_cast<size_t>(v.bx * v.by) * 512u - 448u : 64u;
+  Raw r[8];
+#pragma unroll
+  for (int c = 0; c < 8; ++c) r[c] = __ldg(b + ((c & 1 ? ox : 0u) + (c & 2 ? oy : 0u) + (c & 4 ? oz : 0u)));
+  return blend<Kind>(r, at.fr, policy, tsdf);
 }
 
 // find_zero_crossing's tests of a sample against the previous one
@@ -315,7 +343,6 @@ __device__ __forceinline__ int march_sample(const VolumeDev& v, const SkipDev& s
 // the surface, at the fraction `alpha` from the previous sample to this one;
 // a rise from negative to positive ends the march.
 __device__ __forceinline__ int sample_event(int kind, float tsdf, bool p_have, float p_tsdf, float& alpha) {
-  if (kind == kEnd) return kStop;
   if (kind == kValue && p_have) {
     if (p_tsdf > 0.0f && tsdf <= 0.0f) {
       const float gap = p_tsdf - tsdf;
@@ -387,8 +414,11 @@ __device__ __forceinline__ void box_range(const VolumeDev& v, f3 o, f3 d, float&
   }
 }
 
+// 64 registers (16 CTAs per SM): the rounds are chains of dependent
+// instructions and lookups, so more warps hide more (1001x747 render 0.528 ms
+// at 96 registers, 0.451 at 80, 0.428 at 64 with a few spilled bytes).
 template <int Kind, bool Sparse>
-__global__ void __launch_bounds__(64)
+__global__ void __launch_bounds__(64, 16)
     raycast_kernel(const __grid_constant__ VolumeDev v, SkipDev skip, RaycastParams rp, Intr k, uint32_t width, uint32_t height, Rigid pose, const IcpState* __restrict__ state, float* __restrict__ points) {
   if (state != nullptr) {
     if (state->failed) return;
@@ -451,6 +481,7 @@ __global__ void __launch_bounds__(64)
     while (ray_length < t_in && ray_length <= rp.max_depth) ray_length += base_step;
   }
   float spec = free_step;  // the step the ray's last sample implies
+  bool steady = false;     // the ray's last two samples implied the same step
   // The step after a sample (find_zero_crossing's advance, raycasting.hpp:
   // 204-209): nullopt and non-positive values take the base step.
   auto step_after = [&](int kind, float tsdf) {
@@ -461,9 +492,9 @@ __global__ void __launch_bounds__(64)
     return base_step;
   };
   // Take a sample (known kind and event) into the march state; a decided
-  // sample whose brick holds only its class also takes every following
-  // sample up to the exit of the cube of bricks of that class around it.
-  auto apply = [&](int event, int kind, float tsdf, float r, uint32_t jump, uint32_t radius, float alpha, float p_r) {
+  // sample inside a box of bricks of its class also takes every following
+  // sample up to the box's exit.
+  auto apply = [&](int event, int kind, float tsdf, float r, uint32_t box, uint32_t lowest, float alpha, float p_r) {
     if (event != kNone) {
       done = true;
       if (event == kFound) {
@@ -476,16 +507,17 @@ __global__ void __launch_bounds__(64)
     }
     const float step = step_after(kind, tsdf);
     float last = r, next = r + step;
-    if (jump != 0u) {
-      const uint32_t bxi = jump & 1023u, byi = (jump >> 10) & 1023u, bzi = (jump >> 20) & 1023u;
-      const float t_exit = box_exit(v, g0, inv_gdir, 8u * (bxi - radius), 8u * (byi - radius), 8u * (bzi - radius),
-                                    8u * (2u * radius + 1u), kind == kValue, margin);
+    if (box != 0u) {
+      const float t_exit = box_exit(v, g0, inv_gdir, 8u * (lowest & 1023u), 8u * ((lowest >> 10) & 1023u),
+                                    8u * (lowest >> 20), 8u * box, kind == kValue, margin);
       replay_steps(step, t_exit, rp.max_depth, t_out, last, next);
     }
     have_prev = kind == kValue;
     prev_tsdf = tsdf;
     prev_r = last;
     ray_length = next;
+    // after a negative value the next sample may end the march: no run
+    steady = step == spec && !(tsdf < 0.0f);
     spec = step;
   };
 
@@ -493,27 +525,43 @@ __global__ void __launch_bounds__(64)
   unsigned live;
   while ((live = __ballot_sync(0xFFFFFFFFu, !done)) != 0u) {
     const int n = __popc(live);
-    if (n > rp.coop_rays) {
-      // every live lane takes the next sample of its own ray
+    const int calm = __popc(__ballot_sync(0xFFFFFFFFu, !done && steady));
+    if (n > kCoopLanes || calm != n) {
+      // Every live lane takes up to rp.run decided samples of its own ray, then
+      // one from the corners where it met one: a run of decided samples costs
+      // a round's bookkeeping and the other lanes' gathers once.
       if (!done) {
-        const float r = ray_length;
-        int kind = kEnd;
-        float tsdf = 0.0f, alpha = 0.0f;
-        uint32_t jump = 0u, radius = 0u;
-        if (r <= rp.max_depth && !(r > t_out)) {
-          kind = march_sample<Kind, Sparse>(v, skip, rp.policy, pose.t + (dir * r), tsdf, jump, radius);
+        int cls = kOne;
+        Spot at;
+        f3 point = make(0.0f, 0.0f, 0.0f);
+        for (int i = 0; i < rp.run; ++i) {
+          if (!(ray_length <= rp.max_depth) || ray_length > t_out) {
+            done = true;
+            break;
+          }
+          point = pose.t + (dir * ray_length);
+          cls = decide<Sparse>(v, skip, point, at);
+          if (cls == kGather || cls == kRare) break;
+          // 1.0 after a negative value ends the march (sample_event)
+          if (cls == kOne && have_prev && prev_tsdf < 0.0f) {
+            done = true;
+            break;
+          }
+          apply(kNone, cls == kOne ? kValue : kNull, 1.0f, ray_length, at.box, at.lowest, 0.0f, prev_r);
         }
-        const int event = sample_event(kind, tsdf, have_prev, prev_tsdf, alpha);
-        apply(event, kind, tsdf, r, jump, radius, alpha, prev_r);
+        if (!done && (cls == kGather || cls == kRare)) {
+          float tsdf = 0.0f, alpha = 0.0f;
+          const int kind = resolve<Kind, Sparse>(v, skip, rp.policy, point, cls, at, tsdf);
+          const int event = sample_event(kind, tsdf, have_prev, prev_tsdf, alpha);
+          apply(event, kind, tsdf, ray_length, 0u, 0u, alpha, prev_r);
+        }
       }
       continue;
     }
-    // Few rays left: each live ray gets a segment of G lanes, lane `off` of
-    // which takes the sample `off` steps ahead, assuming every step until
-    // then equals the ray's last one.  The samples up to the first one that
-    // ends the march or takes another step are exactly the march's next
-    // samples; the ray takes them all in this round.
-    const int lg = n > 8 ? 1 : (n > 4 ? 2 : (n > 2 ? 3 : (n > 1 ? 4 : 5)));
+    // Few rays left, all in runs: each live ray gets a segment of G lanes,
+    // lane `off` of which looks at the sample `off` steps ahead, assuming
+    // every step until then equals the ray's last one.
+    const int lg = (n > 4 ? 2 : (n > 2 ? 3 : (n > 1 ? 4 : 5)));
     const unsigned G = 1u << lg;
     const unsigned seg = lane >> lg, off = lane & (G - 1u);
     const bool active = seg < static_cast<unsigned>(n);
@@ -528,44 +576,38 @@ __global__ void __launch_bounds__(64)
     const float o_tout = __shfl_sync(0xFFFFFFFFu, t_out, owner);
     const f3 o_dir = make(__shfl_sync(0xFFFFFFFFu, dir.x, owner), __shfl_sync(0xFFFFFFFFu, dir.y, owner),
                           __shfl_sync(0xFFFFFFFFu, dir.z, owner));
-    const bool o_hp = __shfl_sync(0xFFFFFFFFu, have_prev ? 1 : 0, owner) != 0;
-    const float o_pt = __shfl_sync(0xFFFFFFFFu, prev_tsdf, owner);
-    const float o_pr = __shfl_sync(0xFFFFFFFFu, prev_r, owner);
-    float r = o_r;
-    for (unsigned i = 0; i < off; ++i) r += o_s;
-    int kind = kEnd;
-    float tsdf = 0.0f, alpha = 0.0f;
-    uint32_t jump = 0u, radius = 0u;
-    if (active && r <= rp.max_depth && !(r > o_tout)) {
-      kind = march_sample<Kind, Sparse>(v, skip, rp.policy, pose.t + (o_dir * r), tsdf, jump, radius);
+    // `off` additions of o_s: one multiply inside a binade (replay_steps)
+    float r;
+    {
+      const float second = o_r + o_s, c = second - o_r;
+      const float half_ulp = __uint_as_float(__float_as_uint(o_r) & 0x7F800000u) * 5.9604645e-8f;
+      r = o_r + static_cast<float>(off) * c;
+      if (!(o_r + 32.0f * o_s < 3.3554432e7f * half_ulp && fabsf(o_s - c) < half_ulp && c >= 4.0f * half_ulp)) {
+        r = o_r;
+        for (unsigned i = 0; i < off; ++i) r += o_s;
+      }
     }
-    // the state before this sample: the previous lane's sample, or the ray's
-    const int up_kind = __shfl_up_sync(0xFFFFFFFFu, kind, 1);
-    const float up_tsdf = __shfl_up_sync(0xFFFFFFFFu, tsdf, 1);
-    const float up_r = __shfl_up_sync(0xFFFFFFFFu, r, 1);
-    const float p_r = off == 0 ? o_pr : up_r;
-    const int event = off == 0 ? sample_event(kind, tsdf, o_hp, o_pt, alpha)
-                               : sample_event(kind, tsdf, up_kind == kValue, up_tsdf, alpha);
-    const bool stop = !active || event != kNone || !(step_after(kind, tsdf) == o_s);
-    const unsigned stops = __ballot_sync(0xFFFFFFFFu, stop);
-    // each live lane reads the last sample its segment took
-    unsigned src = lane;
-    if (!done) {
-      const unsigned base = static_cast<unsigned>(__popc(live & ((1u << lane) - 1u))) << lg;
-      const unsigned mine = (stops >> base) & (G == 32u ? 0xFFFFFFFFu : ((1u << G) - 1u));
-      src = base + (mine != 0u ? static_cast<unsigned>(__ffs(mine) - 1) : G - 1u);
-    }
-    const uint32_t m_code = __shfl_sync(
-        0xFFFFFFFFu, static_cast<uint32_t>(event) | (static_cast<uint32_t>(kind) << 2) | (radius << 4), src);
+    int seen = kRare;
+    Spot spot;
+    spot.box = 0u;
+    if (active && r <= rp.max_depth && !(r > o_tout)) seen = decide<Sparse>(v, skip, pose.t + (o_dir * r), spot);
+    // The samples up to the first one that takes another step, or up to
+    // before the first one that needs the corners or ends the march, are
+    // exactly the march's next samples: the ray takes them all.
+    const bool decided = seen == kOne || seen == kNullopt;
+    const unsigned stops = __ballot_sync(0xFFFFFFFFu, !decided || (seen == kOne ? free_step : base_step) != o_s);
+    const unsigned others = __ballot_sync(0xFFFFFFFFu, !decided);
+    const unsigned base = static_cast<unsigned>(__popc(live & ((1u << lane) - 1u))) << lg;
+    const unsigned mine = (stops >> (base & 31u)) & (G == 32u ? 0xFFFFFFFFu : ((1u << G) - 1u));
+    int last = mine != 0u ? __ffs(static_cast<int>(mine)) - 1 : static_cast<int>(G) - 1;
+    if (mine != 0u && ((others >> ((base + last) & 31u)) & 1u)) --last;
+    const bool take = !done && last >= 0;
+    const unsigned src = take ? base + static_cast<unsigned>(last) : lane;
+    const uint32_t code = __shfl_sync(0xFFFFFFFFu, static_cast<uint32_t>(seen) | (spot.box << 2), src);
     const float m_r = __shfl_sync(0xFFFFFFFFu, r, src);
-    const float m_tsdf = __shfl_sync(0xFFFFFFFFu, tsdf, src);
-    const uint32_t m_jump = __shfl_sync(0xFFFFFFFFu, jump, src);
-    const float m_alpha = __shfl_sync(0xFFFFFFFFu, alpha, src);
-    const float m_pr = __shfl_sync(0xFFFFFFFFu, p_r, src);
-    if (!done) {
-      apply(static_cast<int>(m_code & 3u), static_cast<int>((m_code >> 2) & 3u), m_tsdf, m_r, m_jump, m_code >> 4,
-            m_alpha, m_pr);
-    }
+    const uint32_t m_lowest = __shfl_sync(0xFFFFFFFFu, spot.lowest, src);
+    if (take) apply(kNone, (code & 3u) == kOne ? kValue : kNull, 1.0f, m_r, code >> 2, m_lowest, 0.0f, prev_r);
+    steady = steady && take;  // else the ray's next sample is an ordinary round's
   }
   if (!in_image) return;
   f3 surface = nan3();
@@ -890,7 +932,7 @@ void launch_typed(const Pipeline& p, const kf_raycast_camera& cam, float* points
   const uint64_t rays = static_cast<uint64_t>(cam.width) * cam.height;
   const uint32_t lanes = p.raycast_lanes[rays <= 20000u ? 0 : (rays <= 80000u ? 1 : 2)];
   rp.rays_per_warp = p.config.raycast_backend == KF_RAYCAST_BAND_MARCH ? 32u : 32u / lanes;
-  rp.coop_rays = rp.rays_per_warp < 32u ? kCoopLanes : 0;
+  rp.run = rp.rays_per_warp == 32u ? kRunFull : kRunFew;
   dim3 block(p.raycast_block_x, p.raycast_block_y);
   dim3 grid(ceil_div(cam.width, block.x), ceil_div(cam.height, block.y));
   if (rp.rays_per_warp < 32u) {
@@ -908,9 +950,16 @@ void launch_typed(const Pipeline& p, const kf_raycast_camera& cam, float* points
   } else {
     // the dense skip structures exist once an integration prepared them
     const bool dense_skip = p.view.table == nullptr && p.brick_class.count != 0;
-    const SkipDev skip{dense_skip ? p.voxel_bits.ptr : nullptr,
-                       dense_skip ? reinterpret_cast<const uint4*>(p.stencil_bits.ptr) : nullptr,
-                       p.brick_class.ptr, p.brick_radius.ptr, p.null_bricks.ptr};
+    SkipDev skip{};
+    skip.voxel_bits = dense_skip ? p.voxel_bits.ptr : nullptr;
+    skip.stencil_bits = dense_skip ? reinterpret_cast<const uint4*>(p.stencil_bits.ptr) : nullptr;
+    skip.brick_code = p.brick_code.ptr;
+    skip.null_bricks = p.null_bricks.ptr;
+    for (int l = 0; l < 2; ++l) {
+      skip.null_cells[l] = p.null_cells[l].ptr;
+      skip.cells_x[l] = null_cells_along(p.view.bx, l);
+      skip.cells_y[l] = null_cells_along(p.view.by, l);
+    }
     if (p.view.table != nullptr) {
       raycast_kernel<Kind, true><<<grid, block, 0, s>>>(p.view, skip, rp, intr_from(cam.intrinsics), cam.width,
                                                         cam.height, pose, state, points);
