@@ -250,6 +250,7 @@ kf_status kf_pipeline_create(const kf_pipeline_config* config, kf_pipeline** out
         require(entries <= (1ull << 32), "Sparse block capacity out of range");
         p.block_table.resize(entries);
         p.null_bricks.resize(blocks);
+        p.block_slots.resize(blocks);
         for (int l = 0; l < 2; ++l) {
           p.null_cells[l].resize(static_cast<size_t>(null_cells_along((g.res_x + 7) / 8, l)) *
                                  null_cells_along((g.res_y + 7) / 8, l) * null_cells_along((g.res_z + 7) / 8, l));
@@ -266,6 +267,7 @@ kf_status kf_pipeline_create(const kf_pipeline_config* config, kf_pipeline** out
       v.voxels = p.voxels.ptr;
       v.colors = c.color == KF_COLOR_FLOAT ? p.colors.ptr : nullptr;
       v.table = c.storage == KF_STORAGE_SPARSE ? p.block_table.ptr : nullptr;
+      v.slots = c.storage == KF_STORAGE_SPARSE ? p.block_slots.ptr : nullptr;
       v.table_mask = c.storage == KF_STORAGE_SPARSE ? static_cast<uint32_t>(p.block_table.count - 1) : 0u;
       v.rx = g.res_x;
       v.ry = g.res_y;

@@ -163,6 +163,10 @@ struct VolumeDev {
   // dense storage
   const unsigned long long* table;
   uint32_t table_mask;  // entries - 1 (entries a power of two)
+  // and the same map as an array over all blocks (kUnallocated where none),
+  // for kernels that resolve many voxels per thread: one load instead of a
+  // probe sequence
+  const uint32_t* slots;
   uint32_t rx, ry, rz;
   uint32_t bx, by, bz;  // block extent
   float voxel_size;
@@ -225,7 +229,7 @@ __device__ __forceinline__ long long storage_index(const VolumeDev& v, uint32_t 
   if (v.table == nullptr) {
     return static_cast<long long>(block) * 512 + brick_offset(x, y, z);
   }
-  const uint32_t slot = block_table_lookup(v.table, v.table_mask, block);
+  const uint32_t slot = __ldg(v.slots + block);
   if (slot == kUnallocated) return -1;
   return static_cast<long long>(slot) * 512 + brick_offset(x, y, z);
 }

@@ -282,7 +282,7 @@ __global__ void __launch_bounds__(kBlockThreads, 10)
   for (unsigned item = blockIdx.x; item < n; item += gridDim.x) {
     const uint32_t block = list[item];
     // sparse volumes: listed blocks are allocated (SparseVolumeView::find_voxel)
-    const uint32_t slot = v.table != nullptr ? block_table_lookup(v.table, v.table_mask, block) : block;
+    const uint32_t slot = v.table != nullptr ? v.slots[block] : block;
     const uint32_t bxi = block % v.bx, byi = (block / v.bx) % v.by, bzi = block / (v.bx * v.by);
     if (threadIdx.x < 16) {
       s_fused[threadIdx.x] = 0u;
@@ -666,8 +666,8 @@ __global__ void band_compact_kernel(const uint32_t* __restrict__ bits, uint32_t 
 constexpr int kAllocWords = 1024;  // words per CTA of the allocation scan
 
 // Marked blocks not allocated yet, and their count per word.
-__global__ void sparse_new_kernel(const uint32_t* __restrict__ marked, const unsigned long long* __restrict__ table,
-                                  uint32_t table_mask, uint32_t words, uint32_t* __restrict__ new_bits,
+__global__ void sparse_new_kernel(const uint32_t* __restrict__ marked, const uint32_t* __restrict__ block_slots,
+                                  uint32_t words, uint32_t* __restrict__ new_bits,
                                   uint32_t* __restrict__ counts, const IcpState* __restrict__ state) {
   if (state != nullptr && state->failed) return;
   const uint32_t w = blockIdx.x * blockDim.x + threadIdx.x;
@@ -676,7 +676,7 @@ __global__ void sparse_new_kernel(const uint32_t* __restrict__ marked, const uns
   while (m != 0u) {
     const uint32_t b = static_cast<uint32_t>(__ffs(m) - 1);
     m &= m - 1u;
-    if (block_table_lookup(table, table_mask, w * 32u + b) == kUnallocated) fresh |= 1u << b;
+    if (block_slots[w * 32u + b] == kUnallocated) fresh |= 1u << b;
   }
   new_bits[w] = fresh;
   counts[w] = static_cast<uint32_t>(__popc(fresh));
@@ -766,7 +766,8 @@ __global__ void sparse_assign_kernel(const uint32_t* __restrict__ marked, const 
                                      const uint32_t* __restrict__ prefix, const uint32_t* __restrict__ cta_prefix,
                                      uint32_t words, const unsigned long long* __restrict__ allocated,
                                      unsigned long long capacity, unsigned long long* __restrict__ table,
-                                     uint32_t table_mask, uint32_t* __restrict__ slot_block, uint32_t* __restrict__ list,
+                                     uint32_t table_mask, uint32_t* __restrict__ slot_block,
+                                     uint32_t* __restrict__ block_slots, uint32_t* __restrict__ list,
                                      unsigned* __restrict__ count, uint8_t* __restrict__ null_bricks,
                                      uint8_t* __restrict__ null4, uint8_t* __restrict__ null16, uint32_t bx,
                                      uint32_t by, uint32_t bz, const IcpState* __restrict__ state) {
@@ -792,6 +793,7 @@ __global__ void sparse_assign_kernel(const uint32_t* __restrict__ marked, const 
       }
       granted |= 1u << b;
       slot_block[slot] = block;
+      block_slots[block] = static_cast<uint32_t>(slot);
       // the stencils that can reach this block are no longer all nullopt
       const int x = static_cast<int>(block % bx), y = static_cast<int>((block / bx) % by),
                 z = static_cast<int>(block / (bx * by));
@@ -921,6 +923,7 @@ void reset_blocks(Pipeline& p, cudaStream_t s) {
 void reset_sparse(Pipeline& p, cudaStream_t s) {
   if (p.block_table.count == 0) return;
   check(cudaMemsetAsync(p.block_table.ptr, 0xFF, p.block_table.bytes(), s), "block table reset");  // kEmptyEntry
+  check(cudaMemsetAsync(p.block_slots.ptr, 0xFF, p.block_slots.bytes(), s), "block slots reset");  // kUnallocated
   check(cudaMemsetAsync(p.null_bricks.ptr, 1, p.null_bricks.bytes(), s), "sparse null bricks reset");
   for (const auto& cells : p.null_cells) {
     check(cudaMemsetAsync(cells.ptr, 1, cells.bytes(), s), "sparse null cells reset");
@@ -969,7 +972,7 @@ void launch_integrate(Pipeline& p, const float4* table, uint32_t width, uint32_t
     if (p.view.table != nullptr) {
       // sparse: allocate the newly marked blocks, list the allocated ones
       const uint32_t ctas = ceil_div(words, static_cast<uint32_t>(kAllocWords));
-      sparse_new_kernel<<<ceil_div(words, 256), 256, 0, s>>>(p.band_bits.ptr, p.block_table.ptr, p.view.table_mask,
+      sparse_new_kernel<<<ceil_div(words, 256), 256, 0, s>>>(p.band_bits.ptr, p.block_slots.ptr,
                                                              words, p.new_bits.ptr, p.word_prefix.ptr, state);
       check(cudaGetLastError(), "sparse_new_kernel launch");
       sparse_scan_local_kernel<<<ctas, kAllocWords, 0, s>>>(p.word_prefix.ptr, words, p.cta_prefix.ptr, state);
@@ -978,7 +981,8 @@ void launch_integrate(Pipeline& p, const float4* table, uint32_t width, uint32_t
       check(cudaGetLastError(), "sparse_scan_top_kernel launch");
       sparse_assign_kernel<<<ceil_div(words, 256), 256, 0, s>>>(
           p.band_bits.ptr, p.new_bits.ptr, p.word_prefix.ptr, p.cta_prefix.ptr, words, p.allocated.ptr,
-          p.sparse_capacity, p.block_table.ptr, p.view.table_mask, p.slot_block.ptr, p.block_list.ptr,
+          p.sparse_capacity, p.block_table.ptr, p.view.table_mask, p.slot_block.ptr, p.block_slots.ptr,
+          p.block_list.ptr,
           p.block_count.ptr, p.null_bricks.ptr, p.null_cells[0].ptr, p.null_cells[1].ptr,
           p.view.bx, p.view.by, p.view.bz, state);
       check(cudaGetLastError(), "sparse_assign_kernel launch");

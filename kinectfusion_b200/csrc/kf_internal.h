@@ -319,6 +319,7 @@ struct Pipeline {
   // (block -> slot, kf_common.cuh block_table_lookup) of 2^k >= 2 x capacity
   // entries, `sparse_capacity` slots in the pools.
   DeviceArray<unsigned long long> block_table;
+  DeviceArray<uint32_t> block_slots;     // slot of each block, kUnallocated where none (VolumeDev::slots)
   DeviceArray<uint32_t> slot_block;      // block of each allocated slot
   DeviceArray<unsigned long long> allocated;  // [0] attempts so far (overflow included), [1] this frame's base
   DeviceArray<uint32_t> new_bits, word_prefix, cta_prefix;

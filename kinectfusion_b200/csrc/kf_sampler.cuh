@@ -49,7 +49,7 @@ struct Sampler {
     if (bx >= 0 && by >= 0 && bz >= 0 && (bx & 7) != 7 && (by & 7) != 7 && (bz & 7) != 7 &&
         bx + 1 < static_cast<int>(v.rx) && by + 1 < static_cast<int>(v.ry) && bz + 1 < static_cast<int>(v.rz)) {
       // All eight corners in one brick: one storage lookup (sparse storage:
-      // one block-table probe; an unallocated block has no corner), fixed
+      // one block-slot lookup; an unallocated block has no corner), fixed
       // offsets from the base voxel, loads issued together, blended in the
       // reference corner order.
       const long long base =
