@@ -425,13 +425,12 @@ kf_status kf_pipeline_autotune(kf_pipeline* pipeline, const uint16_t* frames, ui
 kf_status kf_tracker_create(const kf_icp_options* options, kf_tracker** out);
 kf_status kf_tracker_destroy(kf_tracker* tracker);
 /* Test hook of the bounded device waits (no reference counterpart).  Each
- * ICP level runs as one cooperative kernel whose CTAs meet at a grid barrier
- * once per Gauss-Newton step; every wait there gives up after 250 ms.  This
- * arms the tracker so that the barrier of its next level never completes
- * (its start count is set beyond any count the arrivals reach): the waits
- * run out, the frame
+ * ICP level runs as one cooperative kernel whose CTAs exchange their partial
+ * sums once per Gauss-Newton step; every wait there gives up after 250 ms.
+ * This arms the tracker so that the exchange of its next level never
+ * completes (it waits for tags nobody writes): the waits run out, the frame
  * is marked failed (no integration), and the call that reads the result
- * returns KF_ERR_DEVICE_TIMEOUT and clears the barrier, after which the
+ * returns KF_ERR_DEVICE_TIMEOUT and clears the exchange, after which the
  * tracker runs normally.  Call it with no work of the tracker in flight. */
 kf_status kf_tracker_stall_next_level(kf_tracker* tracker);
 /* Renders the model at `camera` and tracks `live` against it for `iterations`

@@ -673,8 +673,11 @@ kf_status kf_tracker_create(const kf_icp_options* options, kf_tracker** out) {
       t->impl.options = *options;
       t->impl.params = icp_params_from(*options);
       t->impl.state.resize(1);
-      t->impl.partials.resize(2 * static_cast<size_t>(kIcpMaxGrid) * kIcpSlot);
+      t->impl.partials.resize(kIcpScratchFloats);
+      // no packet of the level kernel's exchange carries a tag yet
+      check(cudaMemset(t->impl.partials.ptr, 0, t->impl.partials.bytes()), "tracker scratch init");
       t->impl.staging.resize(1);
+      t->impl.sums.resize(kIcpSlot);
       prepare_icp_kernels();
       check(cudaMemset(t->impl.state.ptr, 0, sizeof(IcpState)), "tracker state init");
       const kf_rigid identity = {{1, 0, 0, 0, 1, 0, 0, 0, 1}, {0, 0, 0}};
@@ -695,11 +698,11 @@ kf_status kf_tracker_destroy(kf_tracker* tracker) {
 kf_status kf_tracker_stall_next_level(kf_tracker* tracker) {
   return guarded([&] {
     require(tracker != nullptr, "kf_tracker_stall_next_level: null tracker");
-    // a start far above any count the arrivals reach: no wait completes
-    const unsigned long long unreachable = 1ull << 62;
+    // the next level waits for tags nobody writes: no wait completes
+    const unsigned stall = 1u;
     check(cudaMemcpy(reinterpret_cast<char*>(tracker->impl.state.ptr) + offsetof(IcpState, barrier) +
-                         offsetof(IcpBarrier, base),
-                     &unreachable, sizeof(unreachable), cudaMemcpyHostToDevice),
+                         offsetof(IcpBarrier, stall),
+                     &stall, sizeof(stall), cudaMemcpyHostToDevice),
           "barrier stall");
   });
 }
@@ -768,15 +771,8 @@ kf_status kf_icp_level(kf_tracker* tracker, const kf_level_view* live, const flo
     Tracker& t = tracker->impl;
     IcpState* st = t.state.ptr;
     cudaStream_t s = 0;  // the legacy stream, ordered with the caller's device maps
-    launch_icp_set_pose(st, *initial_camera_to_world, 1, s);
-    launch_icp_level_begin(st, t.params.damping_lambda, s);
     // the model transform is fixed for the level (IcpIterationTransforms)
-    float model[12];
-    std::memcpy(model, model_world_to_camera->r, 9 * sizeof(float));
-    std::memcpy(model + 9, model_world_to_camera->t, 3 * sizeof(float));
-    check(cudaMemcpyAsync(reinterpret_cast<char*>(st) + offsetof(IcpState, model), model, sizeof(model),
-                          cudaMemcpyHostToDevice, s),
-          "model upload");
+    launch_icp_level_at(st, *initial_camera_to_world, *model_world_to_camera, t.params.damping_lambda, s);
     IcpLevelArgs a;
     a.live_vertices = live->vertices;
     a.live_normals = live->normals;
@@ -809,21 +805,6 @@ kf_status kf_icp_normal_equations(kf_tracker* tracker, const kf_level_view* live
             "kf_icp_normal_equations: null live vertex or normal map");
     Tracker& t = tracker->impl;
     IcpState* st = t.state.ptr;
-    float cam[12], model[12];
-    std::memcpy(cam, camera->r, 9 * sizeof(float));
-    std::memcpy(cam + 9, camera->t, 3 * sizeof(float));
-    std::memcpy(model, model_world_to_camera->r, 9 * sizeof(float));
-    std::memcpy(model + 9, model_world_to_camera->t, 3 * sizeof(float));
-    const int running = kIcpRunning;
-    const unsigned zero = 0;
-    check(cudaMemcpy(reinterpret_cast<char*>(st) + offsetof(IcpState, camera), cam, sizeof(cam),
-                     cudaMemcpyHostToDevice), "camera upload");
-    check(cudaMemcpy(reinterpret_cast<char*>(st) + offsetof(IcpState, model), model, sizeof(model),
-                     cudaMemcpyHostToDevice), "model upload");
-    check(cudaMemcpy(reinterpret_cast<char*>(st) + offsetof(IcpState, status), &running, sizeof(int),
-                     cudaMemcpyHostToDevice), "status upload");
-    check(cudaMemcpy(reinterpret_cast<char*>(st) + offsetof(IcpState, arrived), &zero, sizeof(unsigned),
-                     cudaMemcpyHostToDevice), "ticket reset");
     IcpLevelArgs a;
     a.live_vertices = live->vertices;
     a.live_normals = live->normals;
@@ -834,10 +815,14 @@ kf_status kf_icp_normal_equations(kf_tracker* tracker, const kf_level_view* live
     a.model_width = model_width;
     a.model_height = model_height;
     a.model_intrinsics = intr_from(model_intrinsics);
-    launch_icp_sweep(a, st, t.partials.ptr, t.params, 0);
-    check(cudaMemcpy(t.staging.ptr, st, sizeof(IcpState), cudaMemcpyDeviceToHost), "sums download");
-    std::memcpy(sums, t.staging.ptr->sums, kIcpSums * sizeof(float));
-    *count = t.staging.ptr->count;
+    // the transforms travel with the launch and the last CTA writes the sums
+    // straight into the tracker's page-locked staging: one launch, one wait
+    launch_icp_sweep(a, st, t.partials.ptr, t.params, *camera, *model_world_to_camera, t.sums.ptr, 0);
+    check(cudaStreamSynchronize(0), "normal equations");
+    std::memcpy(sums, t.sums.ptr, kIcpSums * sizeof(float));
+    uint32_t matched;
+    std::memcpy(&matched, t.sums.ptr + kIcpSums, sizeof(matched));
+    *count = matched;
   });
 }
 

@@ -8,8 +8,8 @@
 //     (icp_correspondence.hpp:111-129) per thread;
 //  2. reduces them per warp with register shuffles and per CTA through
 //     shared memory in a fixed order, writing one partial slot per CTA;
-//  3. meets the other CTAs at a bounded grid barrier, combines every slot in
-//     CTA order with Kahan-compensated FP32 sums, and runs the Gauss-Newton/
+//  3. exchanges the slots with the other CTAs as tagged packets, combines
+//     every slot in CTA order with Kahan-compensated FP32 sums, and runs the Gauss-Newton/
 //     LM step of ProjectiveIcpTracker::estimate_with (icp_optimizer.cpp:
 //     208-302) in FP64 on its own copy of the tracker state: stability veto,
 //     damped LDL^T solve, Rodrigues increment, pose composition and the
@@ -333,14 +333,37 @@ struct Stability {
   float condition_number;
 };
 
+// The stability test from the eigenvalues (icp_optimizer.cpp:319-347).  The
+// Jacobi sweeps take one thread about 6.5 us, so a level runs them for its
+// diagnostics once, after its last step, not every step (kf_icp_level of ten
+// steps at 640x480: 0.237 -> 0.136 ms with the step's other changes).
+__device__ __noinline__ Stability spectrum(const float* sums, const IcpParams& p) {
+  Stability s{false, 0.0f, 0.0f};
+  double a[6][6];
+  for (int r = 0; r < 6; ++r)
+    for (int c = 0; c < 6; ++c) a[r][c] = normal_entry(sums, r, c);
+  double eig[6];
+  if (!jacobi6(a, eig)) return s;
+  double lo = eig[0], hi = eig[0];
+  for (int i = 1; i < 6; ++i) {
+    lo = fmin(lo, eig[i]);
+    hi = fmax(hi, eig[i]);
+  }
+  const float mn = static_cast<float>(lo), mx = static_cast<float>(hi);
+  s.min_eigenvalue = mn;
+  if (mn <= 0.0f || mx <= 0.0f) return s;
+  s.condition_number = mx / mn;
+  s.stable = mn >= p.min_system_eigenvalue && s.condition_number <= p.max_condition_number;
+  return s;
+}
+
 // check_system_stability (icp_optimizer.cpp:319-347).  The common
 // well-conditioned case is decided without eigenvalues: with A = L L^T,
 // s = ||L^-1||_F^2 >= ||A^-1||_2, so lambda_min >= 1/s and
 // lambda_max / lambda_min <= ||A||_F * s; when both bounds meet the limits
 // the system is stable.  Any other case computes the spectrum.  `m`
 // receives L^-1 (packed) when A factorises.
-__device__ Stability stability(const float* sums, const IcpParams& p, bool want_values, double (&m)[21],
-                               bool& chol_ok) {
+__device__ Stability stability(const float* sums, const IcpParams& p, double (&m)[21], bool& chol_ok) {
   Stability s{false, 0.0f, 0.0f};
   double fro = 0.0;  // ||A||_F^2 over the full matrix, row-major
 #pragma unroll
@@ -359,7 +382,7 @@ __device__ Stability stability(const float* sums, const IcpParams& p, bool want_
   double rinv[6];
   chol_ok = cholesky_packed(m, rinv);
   if (chol_ok) lower_inverse_packed(m, rinv);
-  if (!want_values && chol_ok) {
+  if (chol_ok) {
     double inv2 = 0.0;
 #pragma unroll
     for (int i = 0; i < 6; ++i) {
@@ -372,22 +395,7 @@ __device__ Stability stability(const float* sums, const IcpParams& p, bool want_
       return s;
     }
   }
-  double a[6][6];
-  for (int r = 0; r < 6; ++r)
-    for (int c = 0; c < 6; ++c) a[r][c] = normal_entry(sums, r, c);
-  double eig[6];
-  if (!jacobi6(a, eig)) return s;
-  double lo = eig[0], hi = eig[0];
-  for (int i = 1; i < 6; ++i) {
-    lo = fmin(lo, eig[i]);
-    hi = fmax(hi, eig[i]);
-  }
-  const float mn = static_cast<float>(lo), mx = static_cast<float>(hi);
-  s.min_eigenvalue = mn;
-  if (mn <= 0.0f || mx <= 0.0f) return s;
-  s.condition_number = mx / mn;
-  s.stable = mn >= p.min_system_eigenvalue && s.condition_number <= p.max_condition_number;
-  return s;
+  return spectrum(sums, p);
 }
 
 __device__ float grow(const IcpParams& p, float l) { return fminf(l * p.lambda_increase, p.max_lambda); }
@@ -519,8 +527,10 @@ __device__ void pose_to_rigid_floats(const double* pose, float* out) {
 }
 
 // One Gauss-Newton / LM step of estimate_with on the combined sums.
+// `tested` (kIcpSums floats, or null) receives the sums the stability test
+// saw, when it ran.
 __device__ __noinline__ void gauss_newton_step(IcpState* st, const float* sums_in, unsigned long long count_in,
-                                  const IcpParams& p, bool want_values) {
+                                               const IcpParams& p, float* tested) {
   const float* sums = sums_in;
   unsigned long long count = count_in;
   st->iterations += 1;
@@ -553,7 +563,10 @@ __device__ __noinline__ void gauss_newton_step(IcpState* st, const float* sums_i
   }
   double inv[21];
   bool chol_ok = false;
-  const Stability stab = stability(sums, p, want_values, inv, chol_ok);
+  if (tested != nullptr) {
+    for (int i = 0; i < kIcpSums; ++i) tested[i] = sums[i];
+  }
+  const Stability stab = stability(sums, p, inv, chol_ok);
   st->min_system_eigenvalue = stab.min_eigenvalue;
   st->condition_number = stab.condition_number;
   if (!stab.stable && !active) {
@@ -592,18 +605,24 @@ __device__ __noinline__ void gauss_newton_step(IcpState* st, const float* sums_i
 }
 
 // One CTA's share of a correspondence sweep: CTA `cta` of `ctas` associates
-// its pixels (Pix per thread and grid step) and writes its partial slot - the
-// 29 sums and, as integer bits in slot kIcpSums, the matched pixel count.
+// its pixels (Pix per thread and grid step) and returns its partial sums,
+// value i on thread i: the 29 sums and, as integer bits in value kIcpSums,
+// the matched pixel count.  `s_live` (or null) keeps the thread's live points
+// and normals in shared memory between the sweeps of a level, six floats per
+// pixel and thread: `fill` reads them from the maps and stores them there,
+// later sweeps read them back.
 template <int Pix>
-__device__ __forceinline__ void sweep_cta(const IcpLevelArgs& a, const Rigid& cam, const Rigid& model,
-                                          const IcpParams& p, unsigned cta, unsigned ctas, float* __restrict__ slot,
-                                          float (&s_warp)[kIcpBlock / 32][kIcpSlot]) {
+__device__ __forceinline__ float sweep_cta(const IcpLevelArgs& a, const Rigid& cam, const Rigid& model,
+                                           const IcpParams& p, unsigned cta, unsigned ctas,
+                                           float (&s_warp)[kIcpBlock / 32][kIcpSlot], float* s_live = nullptr,
+                                           bool fill = true) {
   // acc[0..28]: the 29 sums, acc[29]: matched pixels, acc[30..31]: padding
   float acc[32];
 #pragma unroll
   for (int i = 0; i < 32; ++i) acc[i] = 0.0f;
   const uint32_t pixels = a.live_width * a.live_height;
   const uint32_t stride = ctas * kIcpBlock;
+  float* kept = s_live + threadIdx.x;
   for (uint32_t first = cta * kIcpBlock + threadIdx.x; first < pixels; first += stride * Pix) {
     // Pix pixels per thread, each step of the association issued for all of
     // them before the next, so their memory latencies overlap
@@ -615,8 +634,23 @@ __device__ __forceinline__ void sweep_cta(const IcpLevelArgs& a, const Rigid& ca
       mi[q] = -1;
       src[q] = lnr[q] = make(0.0f, 0.0f, 0.0f);
       if (pix < pixels) {
-        const f3 lv = ldg3(a.live_vertices + static_cast<size_t>(pix) * 3);
-        const f3 ln = ldg3(a.live_normals + static_cast<size_t>(pix) * 3);
+        f3 lv, ln;
+        if (fill) {
+          lv = ldg3(a.live_vertices + static_cast<size_t>(pix) * 3);
+          ln = ldg3(a.live_normals + static_cast<size_t>(pix) * 3);
+          if (s_live != nullptr) {
+            kept[0] = lv.x;
+            kept[kIcpBlock] = lv.y;
+            kept[2 * kIcpBlock] = lv.z;
+            kept[3 * kIcpBlock] = ln.x;
+            kept[4 * kIcpBlock] = ln.y;
+            kept[5 * kIcpBlock] = ln.z;
+          }
+        } else {
+          lv = make(kept[0], kept[kIcpBlock], kept[2 * kIcpBlock]);
+          ln = make(kept[3 * kIcpBlock], kept[4 * kIcpBlock], kept[5 * kIcpBlock]);
+        }
+        kept += 6 * kIcpBlock;
         if (finite3(lv) && finite3(ln)) {
           const f3 source = apply(cam, lv);
           const f3 sim = apply(model, source);
@@ -681,13 +715,13 @@ __device__ __forceinline__ void sweep_cta(const IcpLevelArgs& a, const Rigid& ca
   }
   s_warp[warp][lane] = acc[0];
   __syncthreads();
+  float sum = 0.0f;
   if (threadIdx.x < kIcpSlot) {
-    float sum = 0.0f;
     for (int w = 0; w < kIcpBlock / 32; ++w) sum += s_warp[w][threadIdx.x];
-    // the count travels as integer bits in slot kIcpSums
-    slot[threadIdx.x] = threadIdx.x == kIcpSums ? __uint_as_float(static_cast<unsigned>(sum)) : sum;
-    __threadfence();
+    // the count travels as integer bits in value kIcpSums
+    if (threadIdx.x == kIcpSums) sum = __uint_as_float(static_cast<unsigned>(sum));
   }
+  return sum;
 }
 
 // Shared memory of the combine: the eight segment sums and compensations.
@@ -698,26 +732,20 @@ struct CombineShared {
   unsigned long long count;
 };
 
+constexpr unsigned kIcpPerSegment = (kIcpMaxGrid + kIcpSegments - 1) / kIcpSegments;
+
 // Deterministic Kahan-compensated combine of `ctas` partial slots, by all
-// threads of the CTA: warp g (segment g of kIcpSegments) lane i (sum i)
-// loads value i of slots g, g + kIcpSegments, ... - every load in flight at
-// once, each warp's loads one coalesced row per slot - and compensates over
-// them in slot order; then the segment results of each sum are combined in
-// segment order.  Ends with c.total / c.count valid after a barrier.
-__device__ __forceinline__ void combine_slots(const float* __restrict__ slots, unsigned ctas, CombineShared& c) {
+// threads of the CTA: warp g (segment g of kIcpSegments) lane i (sum i) holds
+// value i of slots g, g + kIcpSegments, ... in v and compensates over them in
+// slot order; then the segment results of each sum are combined in segment
+// order.  Ends with c.total / c.count valid after a barrier.
+__device__ __forceinline__ void combine_values(const float (&v)[kIcpPerSegment], unsigned ctas, CombineShared& c) {
   static_assert(kIcpBlock == kIcpSegments * 32 && kIcpSlot == 32, "one warp per segment, one lane per slot value");
-  constexpr unsigned kPerSegment = (kIcpMaxGrid + kIcpSegments - 1) / kIcpSegments;
   const unsigned i = threadIdx.x & 31u, g = threadIdx.x >> 5;
-  float v[kPerSegment];
-#pragma unroll
-  for (unsigned u = 0; u < kPerSegment; ++u) {
-    const unsigned b = g + kIcpSegments * u;
-    v[u] = b < ctas ? __ldcg(slots + b * kIcpSlot + i) : 0.0f;
-  }
   if (i < kIcpSums) {
     float sum = 0.0f, comp = 0.0f;
 #pragma unroll
-    for (unsigned u = 0; u < kPerSegment; ++u) {
+    for (unsigned u = 0; u < kIcpPerSegment; ++u) {
       if (g + kIcpSegments * u >= ctas) break;
       const float y = v[u] - comp;
       const float t = sum + y;
@@ -729,7 +757,7 @@ __device__ __forceinline__ void combine_slots(const float* __restrict__ slots, u
   } else if (i == kIcpSums) {
     unsigned n = 0;
 #pragma unroll
-    for (unsigned u = 0; u < kPerSegment; ++u) {
+    for (unsigned u = 0; u < kIcpPerSegment; ++u) {
       if (g + kIcpSegments * u >= ctas) break;
       n += __float_as_uint(v[u]);
     }
@@ -738,6 +766,7 @@ __device__ __forceinline__ void combine_slots(const float* __restrict__ slots, u
   __syncthreads();
   if (threadIdx.x < kIcpSums) {
     float sum = 0.0f, comp = 0.0f;
+#pragma unroll
     for (unsigned g2 = 0; g2 < kIcpSegments; ++g2) {
       const float y = (c.seg_sum[g2][threadIdx.x] - c.seg_comp[g2][threadIdx.x]) - comp;
       const float t = sum + y;
@@ -753,6 +782,18 @@ __device__ __forceinline__ void combine_slots(const float* __restrict__ slots, u
   __syncthreads();
 }
 
+// The combine of plain slots written before this CTA arrived last.
+__device__ __forceinline__ void combine_slots(const float* __restrict__ slots, unsigned ctas, CombineShared& c) {
+  const unsigned i = threadIdx.x & 31u, g = threadIdx.x >> 5;
+  float v[kIcpPerSegment];
+#pragma unroll
+  for (unsigned u = 0; u < kIcpPerSegment; ++u) {
+    const unsigned b = g + kIcpSegments * u;
+    v[u] = b < ctas ? __ldcg(slots + b * kIcpSlot + i) : 0.0f;
+  }
+  combine_values(v, ctas, c);
+}
+
 // One sweep per launch, one CTA per SM, Pix live pixels per thread and
 // grid step; the last CTA to arrive (an atomic ticket, no waiting) combines
 // the slots into the state's sums and count and, with Solve, takes the
@@ -761,15 +802,21 @@ __device__ __forceinline__ void combine_slots(const float* __restrict__ slots, u
 template <bool Solve, int Pix>
 __global__ void __launch_bounds__(kIcpBlock, 1)
     icp_iteration_kernel(IcpLevelArgs a, IcpState* __restrict__ st, float* __restrict__ partials, IcpParams p,
-                         int want_values) {
+                         kf_rigid camera, kf_rigid model, float* __restrict__ result) {
   __shared__ int s_flag;
   __shared__ float s_warp[kIcpBlock / 32][kIcpSlot];
   __shared__ CombineShared s_combine;
-  if (threadIdx.x == 0) s_flag = (st->status != kIcpRunning);
-  __syncthreads();
-  if (s_flag) return;
-  sweep_cta<Pix>(a, rigid_load(st->camera), rigid_load(st->model), p, blockIdx.x, gridDim.x,
-                 partials + blockIdx.x * kIcpSlot, s_warp);
+  if constexpr (Solve) {
+    if (threadIdx.x == 0) s_flag = (st->status != kIcpRunning);
+    __syncthreads();
+    if (s_flag) return;
+  }
+  const float sum = sweep_cta<Pix>(a, Solve ? rigid_load(st->camera) : rigid_from(camera),
+                                   Solve ? rigid_load(st->model) : rigid_from(model), p, blockIdx.x, gridDim.x, s_warp);
+  if (threadIdx.x < kIcpSlot) {
+    partials[blockIdx.x * kIcpSlot + threadIdx.x] = sum;
+    __threadfence();
+  }
   __syncthreads();
   if (threadIdx.x == 0) {
     const unsigned ticket = atomicAdd(&st->arrived, 1u);
@@ -779,11 +826,17 @@ __global__ void __launch_bounds__(kIcpBlock, 1)
   if (!s_flag) return;
   __threadfence();
   combine_slots(partials, gridDim.x, s_combine);
+  if constexpr (!Solve) {
+    if (threadIdx.x < kIcpSums) result[threadIdx.x] = s_combine.total[threadIdx.x];
+    if (threadIdx.x == kIcpSums) result[kIcpSums] = __uint_as_float(static_cast<unsigned>(s_combine.count));
+  }
   if (threadIdx.x == 0) {
     st->arrived = 0;
-    for (int i = 0; i < kIcpSums; ++i) st->sums[i] = s_combine.total[i];
-    st->count = s_combine.count;
-    if (Solve) gauss_newton_step(st, s_combine.total, s_combine.count, p, want_values != 0);
+    if constexpr (Solve) {
+      for (int i = 0; i < kIcpSums; ++i) st->sums[i] = s_combine.total[i];
+      st->count = s_combine.count;
+      gauss_newton_step(st, s_combine.total, s_combine.count, p, nullptr);
+    }
   }
 }
 
@@ -840,70 +893,107 @@ __device__ __forceinline__ unsigned long long global_ns() {
   return t;
 }
 
-// A grid-barrier wait gives up after 250 ms (the sweep it waits for takes
-// microseconds), or after kBarrierPolls polls should the timer not advance
-// (the first kBarrierSpinPolls polls back to back, the rest about 100 ns
-// apart).
-constexpr unsigned long long kBarrierWaitNs = 250000000ull;
-constexpr uint32_t kBarrierPolls = 1u << 24;
-constexpr uint32_t kBarrierSpinPolls = 4096u;
+// A wait for the other CTAs' packets gives up after 250 ms (the sweep it
+// waits for takes microseconds), or after kExchangePolls polls should the
+// timer not advance (the first kExchangeSpinPolls polls back to back, the rest
+// about 100 ns apart).
+constexpr unsigned long long kExchangeWaitNs = 250000000ull;
+constexpr uint32_t kExchangePolls = 1u << 24;
+constexpr uint32_t kExchangeSpinPolls = 4096u;
 
-__device__ __forceinline__ unsigned long long load_acquire64(const unsigned long long* p) {
-  unsigned long long v;
-  asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-  return v;
+// A packet of the step exchange: a slot value and the step's tag in one
+// 8-byte word, which a reader sees whole or not at all.
+__device__ __forceinline__ void store_packet(unsigned long long* p, float value, unsigned tag) {
+  const unsigned long long w = (static_cast<unsigned long long>(tag) << 32) | __float_as_uint(value);
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(w) : "memory");
+}
+__device__ __forceinline__ unsigned long long load_packet(const unsigned long long* p) {
+  unsigned long long w;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(w) : "l"(p) : "memory");
+  return w;
 }
 
-// Counting grid barrier, called by thread 0 of every CTA of a cooperative
-// launch (all CTAs resident, so every arrival comes): barrier `index` of a
-// launch whose arrivals started at `base` completes once the count reaches
-// base + (index + 1) * ctas.  An arrival is one fire-and-forget add after a
-// fence; the count only grows, so nothing is cleared between barriers.  A
-// wait that runs out of time, or sees another CTA's give-up, marks the
-// barrier broken and returns false; the kernel then returns and the host
-// reports KF_ERR_DEVICE_TIMEOUT (and clears the barrier).
-__device__ bool grid_barrier(IcpBarrier* b, unsigned long long base, uint32_t index, unsigned ctas) {
-  const unsigned long long target = base + (static_cast<unsigned long long>(index) + 1ull) * ctas;
-  __threadfence();
-  atomicAdd(&b->count, 1ull);
-  const unsigned long long start = global_ns();
-  for (uint32_t poll = 0; poll < kBarrierPolls; ++poll) {
-    if (load_acquire64(&b->count) >= target) {
-      __threadfence();
-      return true;
+// Waits for the packets of step `tag` of every CTA and combines them.  The
+// packets carry the data and its arrival together, so a step needs no grid
+// barrier: one store and the load that finds it, instead of a fence, an
+// arrival, a poll and the slots' loads after it.  Every CTA of a cooperative
+// launch is resident, so every packet comes; a wait that runs out of time, or
+// sees another CTA's give-up, marks the exchange broken and returns false on
+// every thread; the kernel then returns and the host reports
+// KF_ERR_DEVICE_TIMEOUT.
+__device__ __forceinline__ bool exchange_slots(const unsigned long long* packets, unsigned ctas, unsigned tag,
+                                               IcpBarrier* b, CombineShared& c) {
+  const unsigned i = threadIdx.x & 31u, g = threadIdx.x >> 5;
+  float v[kIcpPerSegment];
+  unsigned missing = 0u;  // bit u: slot g + kIcpSegments * u has not come yet (warp-uniform)
+#pragma unroll
+  for (unsigned u = 0; u < kIcpPerSegment; ++u) {
+    v[u] = 0.0f;
+    if (g + kIcpSegments * u < ctas) missing |= 1u << u;
+  }
+  bool gave_up = false;
+  unsigned long long start = 0;
+  for (uint32_t poll = 0; missing != 0u; ++poll) {
+    unsigned long long w[kIcpPerSegment];
+#pragma unroll
+    for (unsigned u = 0; u < kIcpPerSegment; ++u) {
+      if ((missing >> u) & 1u) w[u] = load_packet(packets + (g + kIcpSegments * u) * kIcpSlot + i);
     }
-    if ((poll & 63u) == 63u) {
-      if (load_acquire(&b->broken) != 0u) return false;
-      if (global_ns() - start > kBarrierWaitNs) break;
+#pragma unroll
+    for (unsigned u = 0; u < kIcpPerSegment; ++u) {
+      if (!((missing >> u) & 1u)) continue;
+      const bool here = i > kIcpSums || static_cast<unsigned>(w[u] >> 32) == tag;
+      if (__all_sync(0xFFFFFFFFu, here)) {
+        v[u] = __uint_as_float(static_cast<unsigned>(w[u]));
+        missing &= ~(1u << u);
+      }
+    }
+    if ((poll & 63u) == 63u && missing != 0u) {
+      const unsigned long long now = global_ns();
+      if (start == 0) start = now;
+      gave_up = load_acquire(&b->broken) != 0u || now - start > kExchangeWaitNs || poll >= kExchangePolls;
+      gave_up = __any_sync(0xFFFFFFFFu, gave_up);
+      if (gave_up) break;
     }
     // the waits are microseconds: poll back to back at first, then sleep
-    if (poll >= kBarrierSpinPolls) __nanosleep(100);
+    if (poll >= kExchangeSpinPolls) __nanosleep(100);
   }
-  atomicExch(&b->broken, 1u);
-  return false;
+  if (gave_up && i == 0u) atomicExch(&b->broken, 1u);
+  if (__syncthreads_or(gave_up)) return false;
+  combine_values(v, ctas, c);
+  return true;
 }
 
 // One whole ICP level in one cooperative launch
 // (BasicDeviceCorrespondenceSweep::run_loop, icp_correspondence.cu:397-439,
 // with the sweep of :216-343): with `begin`, the level start; then up to
-// `iterations` Gauss-Newton steps, each a sweep by every CTA, a grid
-// barrier, and the combine plus FP64 step run redundantly by every CTA on
-// its own shared-memory copy of the tracker state (the same inputs in the
-// same order, so every copy takes the same step and no second barrier is
-// needed); then the level end, written back by CTA 0.  The partial slots
-// alternate between two buffers by step parity: a CTA may write step i+1's
-// slot while another still reads step i's.  Every CTA sees the same status
-// and leaves the loop at the same step.  The sweep, the slot layout and the
-// combine are icp_iteration_kernel's, so the steps are bit-identical to a
-// launch per step at the same grid.
+// `iterations` Gauss-Newton steps, each a sweep by every CTA, the exchange of
+// the partial slots, and the combine plus FP64 step run redundantly by every
+// CTA on its own shared-memory copy of the tracker state (the same inputs in
+// the same order, so every copy takes the same step and nothing has to come
+// back); then the level end, written back by CTA 0.  The packets alternate
+// between two buffers by step parity: a CTA may write step i+1's while another
+// still waits for step i's, and cannot reach step i+2 before every CTA has
+// read step i's.  Every CTA sees the same status and leaves the loop at the
+// same step.  The sweep, the slot values and the combine are
+// icp_iteration_kernel's, so the steps are bit-identical to a launch per step
+// at the same grid.
+//
+// A step is a chain of short phases, so what is left is latency: at 640x480
+// 13.6 us a step with a counting grid barrier and the live maps re-read from
+// L2 every sweep, 10.4 us with packets and the live maps in shared memory
+// (sweep 13.1k -> 6.6k cycles, exchange and combine 6.5k -> 6.2k, of which
+// 148 CTAs reading 148 slots each from L2 are 2.5k; at 320x240, 38 CTAs, the
+// exchange is 3.7k).
 template <int Pix>
 __global__ void __launch_bounds__(kIcpBlock, 1)
     icp_level_kernel(IcpLevelArgs a, IcpState* __restrict__ st, float* __restrict__ partials, IcpParams p,
-                     uint32_t iterations, int level, int begin, int want_values) {
-  __shared__ int s_flag;
+                     uint32_t iterations, int level, int begin, int want_values, int keep_live) {
+  extern __shared__ float s_live[];
   __shared__ float s_warp[kIcpBlock / 32][kIcpSlot];
   __shared__ CombineShared s_combine;
   __shared__ IcpState s_st;
+  __shared__ float s_tested[kIcpSums];
   constexpr unsigned kWords = offsetof(IcpState, barrier) / sizeof(unsigned);
   static_assert(offsetof(IcpState, barrier) % sizeof(unsigned) == 0, "state words");
   {
@@ -913,41 +1003,50 @@ __global__ void __launch_bounds__(kIcpBlock, 1)
   }
   __syncthreads();
   if (threadIdx.x == 0 && begin) level_begin(&s_st, p.damping_lambda);
-  // where this launch's barrier arrivals start (set by the previous launch's
-  // CTA 0 after its last barrier, when every CTA of that launch had arrived)
+  if (threadIdx.x == 0) s_tested[0] = kNaN;  // no step has tested its system yet
+  // the first step's tag (set by the previous launch's CTA 0 after its last
+  // exchange, when every CTA of that launch had read it)
   const unsigned long long base = st->barrier.base;
+  const unsigned stall = st->barrier.stall != 0u ? 0x80000000u : 0u;
   __syncthreads();
   const unsigned ctas = gridDim.x;
+  unsigned long long* packets =
+      reinterpret_cast<unsigned long long*>(partials + static_cast<size_t>(kIcpMaxGrid) * kIcpSlot);
   uint32_t steps = 0;
   for (uint32_t it = 0; it < iterations; ++it) {
     if (s_st.status != kIcpRunning) break;
-    float* slots = partials + (it & 1u) * (kIcpMaxGrid * kIcpSlot);
-    sweep_cta<Pix>(a, rigid_load(s_st.camera), rigid_load(s_st.model), p, blockIdx.x, ctas,
-                   slots + blockIdx.x * kIcpSlot, s_warp);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      s_flag = grid_barrier(&st->barrier, base, it, ctas) ? 1 : 0;
-      // a barrier that gave up fails the frame: later levels skip, the
+    unsigned long long* buffer = packets + (it & 1u) * (kIcpMaxGrid * kIcpSlot);
+    const unsigned tag = static_cast<unsigned>(base + it + 1ull);
+    const float sum = sweep_cta<Pix>(a, rigid_load(s_st.camera), rigid_load(s_st.model), p, blockIdx.x, ctas, s_warp,
+                                     keep_live ? s_live : nullptr, !keep_live || it == 0);
+    if (threadIdx.x <= kIcpSums) store_packet(buffer + blockIdx.x * kIcpSlot + threadIdx.x, sum, tag);
+    if (!exchange_slots(buffer, ctas, tag ^ stall, &st->barrier, s_combine)) {
+      // an exchange that gave up fails the frame: later levels skip, the
       // integration does not run, and the host reports the timeout
-      if (!s_flag) st->failed = 1;
+      if (threadIdx.x == 0) st->failed = 1;
+      return;
     }
-    __syncthreads();
-    if (!s_flag) return;
-    combine_slots(slots, ctas, s_combine);
+    if (threadIdx.x < kIcpSums) s_st.sums[threadIdx.x] = s_combine.total[threadIdx.x];
     if (threadIdx.x == 0) {
-      for (int i = 0; i < kIcpSums; ++i) s_st.sums[i] = s_combine.total[i];
       s_st.count = s_combine.count;
-      gauss_newton_step(&s_st, s_combine.total, s_combine.count, p, want_values != 0);
+      gauss_newton_step(&s_st, s_combine.total, s_combine.count, p, want_values ? s_tested : nullptr);
     }
     __syncthreads();
     ++steps;
   }
   if (blockIdx.x != 0) return;
   if (threadIdx.x == 0) {
+    // the diagnostics' eigenvalues are those of the last system tested; the
+    // steps themselves decide stability from bounds (stability)
+    if (want_values && s_tested[0] == s_tested[0]) {
+      const Stability values = spectrum(s_tested, p);
+      s_st.min_system_eigenvalue = values.min_eigenvalue;
+      s_st.condition_number = values.condition_number;
+    }
     level_end(&s_st, level);
-    // every CTA read `base` before its first arrival, so after CTA 0's last
-    // barrier nothing reads it any more
-    if (steps != 0u) st->barrier.base = base + static_cast<unsigned long long>(steps) * ctas;
+    // every CTA read `base` before its first packet, so after CTA 0's last
+    // exchange nothing reads it any more
+    if (steps != 0u) st->barrier.base = base + steps;
   }
   __syncthreads();
   const unsigned* src = reinterpret_cast<const unsigned*>(&s_st);
@@ -963,8 +1062,7 @@ __global__ void icp_level_end_kernel(IcpState* st, int level) {
   if (threadIdx.x == 0) level_end(st, level);
 }
 
-__global__ void icp_set_pose_kernel(IcpState* st, kf_rigid pose, int reset_frame) {
-  if (threadIdx.x != 0) return;
+__device__ void set_pose(IcpState* st, const kf_rigid& pose, int reset_frame) {
   for (int i = 0; i < 3; ++i) {
     for (int j = 0; j < 3; ++j) st->pose[i * 4 + j] = static_cast<double>(pose.r[i * 3 + j]);
     st->pose[i * 4 + 3] = static_cast<double>(pose.t[i]);
@@ -980,6 +1078,20 @@ __global__ void icp_set_pose_kernel(IcpState* st, kf_rigid pose, int reset_frame
       st->level_correspondences[l] = 0;
     }
   }
+}
+
+__global__ void icp_set_pose_kernel(IcpState* st, kf_rigid pose, int reset_frame) {
+  if (threadIdx.x == 0) set_pose(st, pose, reset_frame);
+}
+
+// kf_icp_level's start: the pose, the level start (icp_level_begin_kernel),
+// and the given model transform in place of the pose's inverse.
+__global__ void icp_level_at_kernel(IcpState* st, kf_rigid pose, kf_rigid model, float damping_lambda) {
+  if (threadIdx.x != 0) return;
+  set_pose(st, pose, 1);
+  level_begin(st, damping_lambda);
+  for (int i = 0; i < 9; ++i) st->model[i] = model.r[i];
+  for (int i = 0; i < 3; ++i) st->model[9 + i] = model.t[i];
 }
 
 }  // namespace
@@ -1012,6 +1124,12 @@ unsigned icp_grid_for(uint32_t pixels) {
 
 namespace {
 
+// Shared memory of the live points and normals a level kernel's CTA keeps
+// between its sweeps: 12 KB per pixel of a thread, at most 16 of them (1.2
+// million live pixels at 148 CTAs; larger images re-read the maps).
+constexpr unsigned kIcpLiveBytes = 6 * kIcpBlock * sizeof(float);
+constexpr unsigned kIcpLiveSteps = 16;
+
 // Largest cooperative grid of icp_level_kernel per device (all CTAs
 // resident at once), set by prepare_icp_kernels.
 constexpr int kMaxIcpDevices = 64;
@@ -1029,7 +1147,11 @@ int current_device() {
 void prepare_icp_kernels() {
   const int device = current_device();
   int per_sm = 0, sms = 0;
-  check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, icp_level_kernel<kIcpPixels>, kIcpBlock, 0),
+  check(cudaFuncSetAttribute(icp_level_kernel<kIcpPixels>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             kIcpLiveSteps * kIcpLiveBytes),
+        "icp level kernel shared memory");
+  check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, icp_level_kernel<kIcpPixels>, kIcpBlock,
+                                                      kIcpLiveSteps * kIcpLiveBytes),
         "icp level kernel occupancy");
   check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device), "SM count");
   const long cap = static_cast<long>(per_sm) * sms;
@@ -1043,9 +1165,10 @@ void launch_icp_level_begin(IcpState* state, float damping_lambda, cudaStream_t 
 }
 
 void launch_icp_sweep(const IcpLevelArgs& args, IcpState* state, float* partials, const IcpParams& params,
-                      cudaStream_t s) {
+                      const kf_rigid& camera, const kf_rigid& model, float* result, cudaStream_t s) {
   const uint32_t pixels = args.live_width * args.live_height;
-  icp_iteration_kernel<false, kIcpPixels><<<icp_grid_for(pixels), kIcpBlock, 0, s>>>(args, state, partials, params, 0);
+  icp_iteration_kernel<false, kIcpPixels>
+      <<<icp_grid_for(pixels), kIcpBlock, 0, s>>>(args, state, partials, params, camera, model, result);
   check(cudaGetLastError(), "icp_iteration_kernel launch");
 }
 
@@ -1055,8 +1178,8 @@ void launch_icp_level_steps(const IcpLevelArgs& args, IcpState* state, float* pa
   check(cudaGetLastError(), "icp_level_begin launch");
   const uint32_t pixels = args.live_width * args.live_height;
   for (uint32_t i = 0; i < iterations; ++i) {
-    icp_iteration_kernel<true, kIcpPixels><<<icp_grid_for(pixels), kIcpBlock, 0, s>>>(args, state, partials, params,
-                                                                                       0);
+    icp_iteration_kernel<true, kIcpPixels>
+        <<<icp_grid_for(pixels), kIcpBlock, 0, s>>>(args, state, partials, params, kf_rigid{}, kf_rigid{}, nullptr);
   }
   check(cudaGetLastError(), "icp_iteration_kernel launch");
   icp_level_end_kernel<<<1, 32, 0, s>>>(state, level);
@@ -1072,7 +1195,9 @@ void launch_icp_level(const IcpLevelArgs& args, IcpState* state, float* partials
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(kIcpBlock);
-  cfg.dynamicSmemBytes = 0;
+  const uint32_t steps = ceil_div(args.live_width * args.live_height, grid * kIcpBlock);
+  const int keep_live = steps <= kIcpLiveSteps ? 1 : 0;
+  cfg.dynamicSmemBytes = keep_live ? steps * kIcpLiveBytes : 0;
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;
@@ -1080,17 +1205,25 @@ void launch_icp_level(const IcpLevelArgs& args, IcpState* state, float* partials
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   check(cudaLaunchKernelEx(&cfg, icp_level_kernel<kIcpPixels>, args, state, partials, params, iterations, level, begin,
-                           want_values),
+                           want_values, keep_live),
         "icp_level_kernel launch");
 }
 
 void check_icp_barrier(const IcpState& host, IcpState* device, cudaStream_t s) {
   if (host.barrier.broken == 0u) return;
-  check(cudaMemsetAsync(reinterpret_cast<char*>(device) + offsetof(IcpState, barrier), 0, sizeof(IcpBarrier), s),
+  const IcpBarrier fresh{host.barrier.base + kIcpStepGap, 0u, 0u};
+  check(cudaMemcpyAsync(reinterpret_cast<char*>(device) + offsetof(IcpState, barrier), &fresh, sizeof(fresh),
+                        cudaMemcpyHostToDevice, s),
         "ICP barrier reset");
   check(cudaStreamSynchronize(s), "ICP barrier reset");
   throw DeviceTimeout(
       "ICP level kernel: a grid-barrier wait gave up before every CTA arrived; the frame is marked failed");
+}
+
+void launch_icp_level_at(IcpState* state, const kf_rigid& pose, const kf_rigid& model, float damping_lambda,
+                         cudaStream_t s) {
+  icp_level_at_kernel<<<1, 32, 0, s>>>(state, pose, model, damping_lambda);
+  check(cudaGetLastError(), "icp_level_at launch");
 }
 
 void launch_icp_set_pose(IcpState* state, kf_rigid pose, int reset_frame, cudaStream_t s) {

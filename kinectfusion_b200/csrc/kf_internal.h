@@ -168,16 +168,18 @@ constexpr int kIcpPixels = 1;         // live pixels per thread and grid step of
 constexpr int kIcpMaxGrid = 148;      // one CTA per SM on a 148-SM B200
 constexpr int kIcpRunning = -1;
 
-// Grid barrier of the whole-level ICP kernel: the arrivals of every CTA at
-// every barrier since the tracker's creation (never reset while the barrier
-// completes), the count at which the next launch starts, and a sticky
-// give-up flag set by a wait that ran out of polls.
+// The step exchange of the whole-level ICP kernel: the steps exchanged since
+// the tracker's creation, whose low 32 bits tag the packets of the next one;
+// a sticky give-up flag set by a wait that ran out of time; and the test
+// hook's flag, which makes the next level wait for tags nobody writes.
 struct IcpBarrier {
-  unsigned long long count;
   unsigned long long base;
   unsigned broken;
-  unsigned pad[3];
+  unsigned stall;
 };
+// Steps skipped after a failed exchange, so that packets left behind by it
+// match no later step.
+constexpr unsigned long long kIcpStepGap = 1ull << 24;
 
 // Lives in device memory; one per tracker.  All poses are camera_to_world.
 struct IcpState {
@@ -232,8 +234,11 @@ struct Tracker {
   kf_icp_options options{};
   IcpParams params{};
   DeviceArray<IcpState> state;
-  DeviceArray<float> partials;  // 2 x kIcpMaxGrid x kIcpSlot, scratch of the sweeps
+  // scratch of the sweeps: kIcpMaxGrid x kIcpSlot plain slots, then the level
+  // kernel's two buffers of as many 8-byte packets
+  DeviceArray<float> partials;
   PinnedArray<IcpState> staging;
+  PinnedArray<float> sums;  // kf_icp_normal_equations' result
 };
 
 // Geometry of one correspondence sweep.
@@ -254,14 +259,17 @@ void prepare_icp_kernels();
 // Begin a level: model world_to_camera from the current pose, status running,
 // unless a previous level failed (then the level stays skipped).
 void launch_icp_level_begin(IcpState* state, float damping_lambda, cudaStream_t stream);
-// One correspondence sweep: the state's sums and count at its camera and
-// model transforms (no solve).
+// One correspondence sweep at the given transforms (no solve): the 29 sums
+// and, as integer bits, the match count go to `result`, kIcpSlot floats in
+// device or page-locked host memory.
 void launch_icp_sweep(const IcpLevelArgs& args, IcpState* state, float* partials, const IcpParams& params,
-                      cudaStream_t stream);
+                      const kf_rigid& camera, const kf_rigid& model, float* result, cudaStream_t stream);
+// Floats of a tracker's sweep scratch.
+constexpr size_t kIcpScratchFloats = 5 * static_cast<size_t>(kIcpMaxGrid) * kIcpSlot;
 // A whole level in one cooperative launch: with `begin` the level start,
 // then up to `iterations` Gauss-Newton steps (the loop leaves at the first
 // non-running status), then the level end (level >= 0 records the frame's
-// per-level results).  `partials` holds two sweeps' slots.
+// per-level results).
 void launch_icp_level(const IcpLevelArgs& args, IcpState* state, float* partials, const IcpParams& params,
                       uint32_t iterations, int level, int begin, int want_values, cudaStream_t stream);
 // The same level as launches that need no co-residency: a begin kernel,
@@ -274,6 +282,10 @@ void launch_icp_level_steps(const IcpLevelArgs& args, IcpState* state, float* pa
 // Throws DeviceTimeout when the downloaded state `host` shows a grid barrier
 // that gave up; the device barrier is cleared first (ordered on `stream`).
 void check_icp_barrier(const IcpState& host, IcpState* device, cudaStream_t stream);
+// kf_icp_level's start: the pose, the level start, and the given model
+// transform in place of the pose's inverse.
+void launch_icp_level_at(IcpState* state, const kf_rigid& pose, const kf_rigid& model, float damping_lambda,
+                         cudaStream_t stream);
 // Set the device pose (FP64 + float) from a float rigid transform.
 void launch_icp_set_pose(IcpState* state, kf_rigid pose, int reset_frame, cudaStream_t stream);
 
