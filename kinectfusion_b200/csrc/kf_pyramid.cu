@@ -40,34 +40,100 @@ DepthParams depth_params(const kf_depth_options& o) {
 constexpr int kTileX = 32;
 constexpr int kTileY = 8;
 
-// BilateralFilter::operator() (depth_processing.hpp:71-115).  The Gaussian is
-// exp evaluated in double and rounded once to float: the correctly rounded
-// value of the float exponent, which the CPU oracle computes the same way.
+// The bilateral weight of a float exponent in [-104, 0]: exp evaluated in
+// double and rounded once to float, the correctly rounded value (the CPU
+// oracle computes the same).  Table-driven as in Tang, "Table-driven
+// implementation of the exponential function in IEEE floating-point
+// arithmetic" (1989): x = (32 m + j) ln2 / 32 + r, exp(x) = 2^m 2^(j/32) e^r
+// with e^r from its Taylor series to r^5 (|r| <= ln2 / 64, error below
+// 2^-48).  A result within 2^-45 of a float rounding boundary, and one that
+// rounds to a subnormal float, takes the library's exp instead.
+constexpr int kExpTable = 32;
+__device__ __forceinline__ float gaussian(float arg, const double* s_exp2) {
+  const double x = static_cast<double>(arg);
+  const double shifted = __fma_rn(x, 46.16624130844683, 6755399441055744.0);  // 32 / ln2, 1.5 * 2^52
+  const int k = __double2loint(shifted);
+  const double kd = shifted - 6755399441055744.0;
+  // ln2 / 32 in two parts, the first of 26 bits: kd (13 bits) times it is exact
+  double r = __fma_rn(kd, -0.02166084898635745, x);
+  r = __fma_rn(kd, -4.06140840434059e-10, r);
+  double e = __fma_rn(r, 1.0 / 120.0, 1.0 / 24.0);
+  e = __fma_rn(r, e, 1.0 / 6.0);
+  e = __fma_rn(r, e, 0.5);
+  e = __fma_rn(r, e, 1.0);
+  e = __fma_rn(r, e, 1.0);
+  e *= s_exp2[k & (kExpTable - 1)];
+  const unsigned low = static_cast<unsigned>(__double2loint(e));
+  const double y = __hiloint2double(__double2hiint(e) + ((k >> 5) << 20), static_cast<int>(low));
+  // the 29 bits below a float's last: half way is 2^28
+  if (((low - 0x10000000u + 0x80u) & 0x1FFFFFFFu) < 0x100u || !(arg >= -87.0f)) return static_cast<float>(exp(x));
+  return static_cast<float>(y);
+}
+
+// BilateralFilter::operator() (depth_processing.hpp:71-115).  A CTA stages its
+// pixels and their border of `radius` as metres (NaN where the depth is not
+// usable) and raw values, so each depth is divided and range-tested once
+// instead of once per window it is in.  Bound by its double arithmetic:
+// 640x480 at radius 2, 24.7 us against 29.6 us with exp and a division per
+// sample.
+template <bool Tile>
 __global__ void __launch_bounds__(kTileX* kTileY)
     bilateral_kernel(const uint16_t* __restrict__ in, uint16_t* __restrict__ out, int width,
                      int height, DepthParams p) {
+  extern __shared__ float s_tile[];
+  __shared__ double s_exp2[kExpTable];
+  const int span_x = kTileX + 2 * p.radius, span_y = kTileY + 2 * p.radius;
+  float* s_metres = s_tile;
+  float* s_raw = s_tile + span_x * span_y;
+  const int tid = threadIdx.y * kTileX + threadIdx.x;
+  const int left = static_cast<int>(blockIdx.x) * kTileX - p.radius;
+  const int top = static_cast<int>(blockIdx.y) * kTileY - p.radius;
+  auto pixel = [&](int x, int y, float& m, float& value) {
+    m = kNaN;
+    value = 0.0f;
+    if (x >= 0 && y >= 0 && x < width && y < height) {
+      const uint16_t raw = __ldg(in + y * width + x);
+      value = static_cast<float>(raw);
+      if (!depth_in_range(raw, p.depth_scale, p.min_depth, p.max_depth, m)) m = kNaN;
+    }
+  };
+  if constexpr (Tile) {
+    for (int i = tid; i < span_x * span_y; i += kTileX * kTileY) {
+      pixel(left + i % span_x, top + i / span_x, s_metres[i], s_raw[i]);
+    }
+  }
+  if (tid < kExpTable) s_exp2[tid] = exp2(static_cast<double>(tid) * (1.0 / kExpTable));
+  __syncthreads();
   const int col = blockIdx.x * kTileX + threadIdx.x;
   const int row = blockIdx.y * kTileY + threadIdx.y;
   if (col >= width || row >= height) return;
-  float center;
+  auto staged = [&](int dx, int dy, float& m, float& value) {
+    if constexpr (Tile) {
+      const int i = (static_cast<int>(threadIdx.y) + p.radius + dy) * span_x + static_cast<int>(threadIdx.x) + p.radius + dx;
+      m = s_metres[i];
+      value = s_raw[i];
+    } else {
+      pixel(col + dx, row + dy, m, value);
+    }
+  };
+  float center, unused;
+  staged(0, 0, center, unused);
   uint16_t result = 0;
-  if (depth_in_range(__ldg(in + row * width + col), p.depth_scale, p.min_depth, p.max_depth, center)) {
-    const int x_begin = max(col - p.radius, 0);
-    const int y_begin = max(row - p.radius, 0);
-    const int x_end = min(col + p.radius, width - 1);
-    const int y_end = min(row + p.radius, height - 1);
+  if (center == center) {
     float weighted_sum = 0.0f;
     float weight_sum = 0.0f;
-    for (int y = y_begin; y <= y_end; ++y) {
-      for (int x = x_begin; x <= x_end; ++x) {
-        const uint16_t raw = __ldg(in + y * width + x);
-        float sample;
-        if (!depth_in_range(raw, p.depth_scale, p.min_depth, p.max_depth, sample)) continue;
-        const float d2 = static_cast<float>(((x - col) * (x - col)) + ((y - row) * (y - row)));
+    // pixels outside the image are NaN: skipped, as the reference's clipped window
+    for (int dy = -p.radius; dy <= p.radius; ++dy) {
+      for (int dx = -p.radius; dx <= p.radius; ++dx) {
+        float sample, raw;
+        staged(dx, dy, sample, raw);
+        if (sample != sample) continue;
+        const float d2 = static_cast<float>((dx * dx) + (dy * dy));
         const float dd = sample - center;
         const float arg = (d2 * p.spatial_scale) + (dd * dd * p.range_scale);
-        const float weight = static_cast<float>(exp(static_cast<double>(arg)));
-        weighted_sum += weight * static_cast<float>(raw);
+        if (arg < -104.0f) continue;  // rounds to zero: adds nothing
+        const float weight = gaussian(arg, s_exp2);
+        weighted_sum += weight * raw;
         weight_sum += weight;
       }
     }
@@ -89,24 +155,41 @@ __device__ __forceinline__ f3 vertex_at(const uint16_t* __restrict__ depth, int 
 }
 
 // One level: vertex + NormalEstimation (depth_processing.hpp:251-279) +
-// BlockDownsample into the next level (depth_processing.hpp:153-187).
+// BlockDownsample into the next level (depth_processing.hpp:153-187).  The
+// CTA's vertices and a border of one pixel are projected once, into shared
+// memory, instead of five times per pixel (640x480: 9.0 -> 6.7 us).
 __global__ void __launch_bounds__(kTileX* kTileY)
     level_kernel(const uint16_t* __restrict__ depth, int width, int height, Intr k, DepthParams p,
                  float* __restrict__ vertices, float* __restrict__ normals,
                  uint16_t* __restrict__ next) {
+  constexpr int kSpanX = kTileX + 2, kSpanY = kTileY + 2;
+  __shared__ float s_x[kSpanX * kSpanY], s_y[kSpanX * kSpanY], s_z[kSpanX * kSpanY];
+  const int tid = threadIdx.y * kTileX + threadIdx.x;
+  const int left = static_cast<int>(blockIdx.x) * kTileX - 1, top = static_cast<int>(blockIdx.y) * kTileY - 1;
+  for (int i = tid; i < kSpanX * kSpanY; i += kTileX * kTileY) {
+    const int x = left + i % kSpanX, y = top + i / kSpanX;
+    f3 v = nan3();
+    if (x >= 0 && y >= 0 && x < width && y < height) v = vertex_at(depth, width, x, y, k, p);
+    s_x[i] = v.x;
+    s_y[i] = v.y;
+    s_z[i] = v.z;
+  }
+  __syncthreads();
   const int col = blockIdx.x * kTileX + threadIdx.x;
   const int row = blockIdx.y * kTileY + threadIdx.y;
   if (col >= width || row >= height) return;
-  const f3 c = vertex_at(depth, width, col, row, k, p);
+  const int at = (threadIdx.y + 1) * kSpanX + threadIdx.x + 1;
+  auto vertex = [&](int i) { return make(s_x[i], s_y[i], s_z[i]); };
+  const f3 c = vertex(at);
   const size_t pix = static_cast<size_t>(row) * width + col;
   store3(vertices + pix * 3, c);
 
   f3 n = nan3();
   if (col != 0 && row != 0 && col + 1 < width && row + 1 < height) {
-    const f3 l = vertex_at(depth, width, col - 1, row, k, p);
-    const f3 r = vertex_at(depth, width, col + 1, row, k, p);
-    const f3 t = vertex_at(depth, width, col, row - 1, k, p);
-    const f3 b = vertex_at(depth, width, col, row + 1, k, p);
+    const f3 l = vertex(at - 1);
+    const f3 r = vertex(at + 1);
+    const f3 t = vertex(at - kSpanX);
+    const f3 b = vertex(at + kSpanX);
     if (finite3((((c + l) + r) + t) + b) &&
         !(fabsf(r.z - l.z) > p.max_normal_depth_jump || fabsf(b.z - t.z) > p.max_normal_depth_jump)) {
       const f3 nn = cross(b - t, r - l);
@@ -204,8 +287,16 @@ void Pyramid::launch(cudaStream_t s) const {
         check(cudaMemcpyAsync(b.depth.ptr, raw.ptr, raw.bytes(), cudaMemcpyDeviceToDevice, s),
               "pyramid level-0 copy");
       } else {
-        bilateral_kernel<<<grid, block, 0, s>>>(raw.ptr, b.depth.ptr, static_cast<int>(b.width),
-                                                static_cast<int>(b.height), p);
+        // a window too large for the staging (48 KB) reads its pixels directly
+        const size_t tile = 2 * sizeof(float) * (kTileX + 2 * static_cast<size_t>(options.bilateral_radius)) *
+                            (kTileY + 2 * static_cast<size_t>(options.bilateral_radius));
+        if (tile <= 47u * 1024u) {
+          bilateral_kernel<true><<<grid, block, tile, s>>>(raw.ptr, b.depth.ptr, static_cast<int>(b.width),
+                                                           static_cast<int>(b.height), p);
+        } else {
+          bilateral_kernel<false><<<grid, block, 0, s>>>(raw.ptr, b.depth.ptr, static_cast<int>(b.width),
+                                                         static_cast<int>(b.height), p);
+        }
         check(cudaGetLastError(), "bilateral_kernel launch");
       }
     }
