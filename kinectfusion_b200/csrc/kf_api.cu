@@ -327,7 +327,7 @@ kf_status kf_pipeline_destroy(kf_pipeline* pipeline) {
 }
 
 static void enqueue_reset(Pipeline& p) {
-  launch_fill_volume(p, p.stream);
+  launch_refill_volume(p, p.stream);
   reset_sparse(p, p.stream);
   reset_blocks(p, p.stream);  // the raycast's skip structures describe the volume
   if (p.band_map.count) {
@@ -364,8 +364,7 @@ kf_status kf_pipeline_integrate(kf_pipeline* pipeline, const kf_frame_view* fram
     const float* normals = stage(f.normals, n * 3, f.memory, p.own_normals, p.stream);
     if (p.pixel_table.count != n) p.pixel_table.resize(n);
     const Intr k = intr_from(f.intrinsics);
-    launch_pixel_table(depth, color, normals, f.width, f.height, k, p.config.integration, p.config.tsdf_rule,
-                       p.pixel_table.ptr, p.stream);
+    launch_pixel_table(p, depth, color, normals, f.width, f.height, k, p.pixel_table.ptr, p.stream);
     launch_integrate(p, p.pixel_table.ptr, f.width, f.height, k, rigid_from(f.world_to_camera),
                      color != nullptr, nullptr, p.stream);
     check(cudaStreamSynchronize(p.stream), "integrate");

@@ -54,9 +54,8 @@ void record_frame(Pipeline& p, Pyramid& pyr, Tracker& t, const Pipeline::GraphKe
   if (fork) check(cudaEventRecord(p.pyramid_event, side), "graph fork");
   const PyramidLevelBuffers& l0 = pyr.levels[0];
   const Intr k0 = intr_from(pyr.intrinsics);
-  launch_pixel_table(pyr.raw.ptr, has_color ? p.frame_color.ptr : nullptr, l0.normals.ptr, pyr.width, pyr.height, k0,
-                     p.config.integration, p.config.tsdf_rule, p.pixel_table.ptr, side);
-  launch_integrate_inputs(p, p.pixel_table.ptr, pyr.width, pyr.height, side);
+  launch_pixel_table(p, pyr.raw.ptr, has_color ? p.frame_color.ptr : nullptr, l0.normals.ptr, pyr.width, pyr.height,
+                     k0, p.pixel_table.ptr, side);
   if (fork) check(cudaEventRecord(p.inputs_event, side), "graph join");
   frame_begin_kernel<<<1, 32, 0, s>>>(st);
   check(cudaGetLastError(), "frame_begin launch");
@@ -101,7 +100,7 @@ void record_frame(Pipeline& p, Pyramid& pyr, Tracker& t, const Pipeline::GraphKe
     }
   }
   if (fork) check(cudaStreamWaitEvent(s, p.inputs_event, 0), "graph join");  // also joins the pyramid
-  launch_integrate(p, p.pixel_table.ptr, pyr.width, pyr.height, k0, Rigid{}, has_color, st, s, true);
+  launch_integrate(p, p.pixel_table.ptr, pyr.width, pyr.height, k0, Rigid{}, has_color, st, s);
   check(cudaMemcpyAsync(p.result_staging.ptr, st, sizeof(IcpState), cudaMemcpyDeviceToHost, s), "result download");
 }
 

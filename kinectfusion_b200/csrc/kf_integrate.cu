@@ -41,6 +41,7 @@ struct IntegParams {
 };
 
 constexpr int kTile = 8;          // pixels per depth tile edge
+constexpr int kTableX = 32;       // pixels per row of a pixel-table CTA (kTile rows)
 constexpr int kBlockThreads = 128;
 
 // Per-pixel part of IntegrationContext::observe and the rule weight
@@ -49,13 +50,13 @@ __global__ void pixel_table_kernel(const uint16_t* __restrict__ depth, const uin
                                    const float* __restrict__ normals, uint32_t width, uint32_t height,
                                    Intr k, float depth_scale, float min_depth, float max_depth,
                                    float observation_weight, int angle_weighted,
-                                   float4* __restrict__ table) {
-  const uint32_t col = blockIdx.x * blockDim.x + threadIdx.x;
-  const uint32_t row = blockIdx.y * blockDim.y + threadIdx.y;
-  if (col >= width || row >= height) return;
-  const size_t pix = static_cast<size_t>(row) * width + col;
+                                   float4* __restrict__ table, float* __restrict__ tiles, uint32_t tiles_x) {
+  const uint32_t col = blockIdx.x * kTableX + threadIdx.x;
+  const uint32_t row = blockIdx.y * kTile + threadIdx.y;
+  const bool in_image = col < width && row < height;
+  const size_t pix = in_image ? static_cast<size_t>(row) * width + col : 0;
   float sd;
-  bool valid = depth_in_range(depth[pix], depth_scale, min_depth, max_depth, sd);
+  bool valid = in_image && depth_in_range(depth[pix], depth_scale, min_depth, max_depth, sd);
   const f3 ray = back_project(k, static_cast<float>(col), static_cast<float>(row), 1.0f);
   const float lambda = norm(ray);
   if (!finite3(ray) || lambda == 0.0f) valid = false;
@@ -69,25 +70,28 @@ __global__ void pixel_table_kernel(const uint16_t* __restrict__ depth, const uin
       weight *= cos_theta / sd;
     }
   }
-  const uint32_t c = color != nullptr ? color[pix] : 0u;
-  table[pix] = make_float4(valid ? sd : kNaN, lambda, weight, __uint_as_float(c));
-}
-
-// Level 0 of the depth-tile pyramid: the largest usable depth of each 8x8
-// pixel tile (0 when the tile has none).
-__global__ void tile_max_kernel(const float4* __restrict__ table, uint32_t width, uint32_t height,
-                                uint32_t tiles_x, uint32_t tiles_y, float* __restrict__ out) {
-  const uint32_t tx = blockIdx.x * blockDim.x + threadIdx.x;
-  const uint32_t ty = blockIdx.y * blockDim.y + threadIdx.y;
-  if (tx >= tiles_x || ty >= tiles_y) return;
-  float m = 0.0f;
-  for (uint32_t y = ty * kTile; y < min((ty + 1) * kTile, height); ++y) {
-    for (uint32_t x = tx * kTile; x < min((tx + 1) * kTile, width); ++x) {
-      const float d = __ldg(&table[static_cast<size_t>(y) * width + x].x);
-      if (d > m) m = d;  // NaN compares false
-    }
+  if (in_image) {
+    const uint32_t c = color != nullptr ? color[pix] : 0u;
+    table[pix] = make_float4(valid ? sd : kNaN, lambda, weight, __uint_as_float(c));
   }
-  out[ty * tiles_x + tx] = m;
+  if (tiles == nullptr) return;
+  // Level 0 of the depth-tile pyramid: the largest usable depth of each 8x8
+  // pixel tile (0 when the tile has none); a CTA's row of threads is a pixel
+  // row of four tiles.  (A kernel of its own, a thread per tile walking its 64
+  // pixels, took 12 us at 640x480.)
+  float m = valid ? sd : 0.0f;
+#pragma unroll
+  for (int off = 1; off < kTile; off <<= 1) m = fmaxf(m, __shfl_xor_sync(0xFFFFFFFFu, m, off));
+  __shared__ float s_max[kTile][kTableX / kTile];
+  if (threadIdx.x % kTile == 0) s_max[threadIdx.y][threadIdx.x / kTile] = m;
+  __syncthreads();
+  if (threadIdx.y == 0 && threadIdx.x < kTableX / kTile) {
+    m = s_max[0][threadIdx.x];
+#pragma unroll
+    for (int y = 1; y < kTile; ++y) m = fmaxf(m, s_max[y][threadIdx.x]);
+    const uint32_t tx = blockIdx.x * (kTableX / kTile) + threadIdx.x;
+    if (tx < tiles_x) tiles[blockIdx.y * tiles_x + tx] = m;
+  }
 }
 
 struct TileLevels {
@@ -832,17 +836,77 @@ __global__ void fill_kernel(void* voxels, float4* colors, size_t count) {
   }
 }
 
+// Calls `visit` with the storage slot of every brick that may hold a fused
+// voxel, a warp at a time: dense storage, the bricks with an observed bit
+// (every voxel an integration wrote has one); sparse storage, the slots
+// handed out so far.
+template <typename Visit>
+__device__ __forceinline__ void for_touched_bricks(const uint4* __restrict__ voxel_bits,
+                                                   const unsigned long long* __restrict__ allocated,
+                                                   unsigned long long slots, Visit visit) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const unsigned long long warps = (static_cast<unsigned long long>(gridDim.x) * blockDim.x) >> 5;
+  const unsigned long long warp = (static_cast<unsigned long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+  if (allocated != nullptr) {
+    const unsigned long long used = min(*allocated, slots);
+    for (unsigned long long s = warp; s < used; s += warps) visit(s);
+    return;
+  }
+  for (unsigned long long first = warp * 32u; first < slots; first += warps * 32u) {
+    uint32_t any = 0u;
+    if (first + lane < slots) {
+#pragma unroll
+      for (int z = 0; z < 8; ++z) {
+        const uint4 layer = __ldg(voxel_bits + (first + lane) * 8u + z);
+        any |= layer.z | layer.w;
+      }
+    }
+    for (uint32_t todo = __ballot_sync(0xFFFFFFFFu, any != 0u); todo != 0u; todo &= todo - 1u) {
+      visit(first + static_cast<uint32_t>(__ffs(static_cast<int>(todo)) - 1));
+    }
+  }
+}
+
+// Every touched brick unobserved again: a reset writes what integrations
+// wrote, not the whole volume (384^3 int16 with colour, 10 frames: 30 us
+// against 189 us; the 8.6 GB pool of a 2048^3 sparse domain: 11 us against
+// 1715 us).
 template <int Kind>
-__global__ void count_observed_kernel(const void* voxels, size_t count, unsigned long long* result) {
+__global__ void __launch_bounds__(256)
+    refill_kernel(void* voxels, float4* colors, const uint4* __restrict__ voxel_bits,
+                  const unsigned long long* __restrict__ allocated, unsigned long long slots) {
+  using VT = VoxelTraits<Kind>;
+  auto* out = reinterpret_cast<typename VT::Raw*>(voxels);
+  const uint32_t lane = threadIdx.x & 31u;
+  for_touched_bricks(voxel_bits, allocated, slots, [&](unsigned long long brick) {
+#pragma unroll
+    for (uint32_t i = 0; i < 16u; ++i) out[brick * 512u + i * 32u + lane] = VT::unobserved();
+    if (colors != nullptr) {
+#pragma unroll
+      for (uint32_t i = 0; i < 16u; ++i) {
+        colors[brick * 512u + i * 32u + lane] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      }
+    }
+  });
+}
+
+// Voxels with a weight, in the touched bricks (384^3 int16: 34 us
+// against 93 us over the whole volume).
+template <int Kind>
+__global__ void __launch_bounds__(256)
+    count_observed_kernel(const void* voxels, const uint4* __restrict__ voxel_bits,
+                          const unsigned long long* __restrict__ allocated, unsigned long long slots,
+                          unsigned long long* result) {
   using VT = VoxelTraits<Kind>;
   const auto* in = reinterpret_cast<const typename VT::Raw*>(voxels);
-  const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
+  const uint32_t lane = threadIdx.x & 31u;
   unsigned long long local = 0;
-  for (size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < count; i += stride) {
-    local += VT::weight(in[i]) > 0.0f ? 1u : 0u;
-  }
+  for_touched_bricks(voxel_bits, allocated, slots, [&](unsigned long long brick) {
+#pragma unroll
+    for (uint32_t i = 0; i < 16u; ++i) local += VT::weight(in[brick * 512u + i * 32u + lane]) > 0.0f ? 1u : 0u;
+  });
   for (int off = 16; off > 0; off >>= 1) local += __shfl_xor_sync(0xFFFFFFFFu, local, off);
-  if ((threadIdx.x & 31) == 0 && local) atomicAdd(result, local);
+  if (lane == 0 && local) atomicAdd(result, local);
 }
 
 TileLevels tile_levels_of(const Pipeline& p) {
@@ -931,31 +995,22 @@ void reset_sparse(Pipeline& p, cudaStream_t s) {
   check(cudaMemsetAsync(p.allocated.ptr, 0, p.allocated.bytes(), s), "sparse counter reset");
 }
 
-void launch_pixel_table(const uint16_t* depth, const uint32_t* color, const float* normals, uint32_t width,
-                        uint32_t height, Intr k, const kf_integration_options& o, int rule, float4* table,
-                        cudaStream_t s) {
-  const dim3 block(32, 8);
-  const dim3 grid(ceil_div(width, 32), ceil_div(height, 8));
-  pixel_table_kernel<<<grid, block, 0, s>>>(depth, color, normals, width, height, k, o.depth_scale, o.min_depth,
-                                            o.max_depth, o.observation_weight, rule == KF_RULE_ANGLE_WEIGHTED,
-                                            table);
-  check(cudaGetLastError(), "pixel_table_kernel launch");
-}
-
-void launch_integrate_inputs(Pipeline& p, const float4* table, uint32_t width, uint32_t height, cudaStream_t s) {
+void launch_pixel_table(Pipeline& p, const uint16_t* depth, const uint32_t* color, const float* normals,
+                        uint32_t width, uint32_t height, Intr k, float4* table, cudaStream_t s) {
   prepare_blocks(p, width, height, s);
-  if (p.config.integration.mode == KF_INTEGRATION_BAND) return;
-  // depth-tile pyramid
-  const TileLevels lv = tile_levels_of(p);
-  tile_max_kernel<<<dim3(ceil_div(lv.w[0], 16), ceil_div(lv.h[0], 16)), dim3(16, 16), 0, s>>>(
-      table, width, height, lv.w[0], lv.h[0], p.depth_tiles.ptr);
-  check(cudaGetLastError(), "tile_max_kernel launch");
-  tile_pyramid_kernel<<<1, 1024, 0, s>>>(p.depth_tiles.ptr, lv);
+  const kf_integration_options& o = p.config.integration;
+  const bool tiles = o.mode != KF_INTEGRATION_BAND;  // the full sweep's block culling
+  pixel_table_kernel<<<dim3(ceil_div(width, kTableX), ceil_div(height, kTile)), dim3(kTableX, kTile), 0, s>>>(
+      depth, color, normals, width, height, k, o.depth_scale, o.min_depth, o.max_depth, o.observation_weight,
+      p.config.tsdf_rule == KF_RULE_ANGLE_WEIGHTED, table, tiles ? p.depth_tiles.ptr : nullptr, p.tile_w[0]);
+  check(cudaGetLastError(), "pixel_table_kernel launch");
+  if (!tiles) return;
+  tile_pyramid_kernel<<<1, 1024, 0, s>>>(p.depth_tiles.ptr, tile_levels_of(p));
   check(cudaGetLastError(), "tile_pyramid_kernel launch");
 }
 
 void launch_integrate(Pipeline& p, const float4* table, uint32_t width, uint32_t height, Intr k, Rigid T,
-                      int has_color, const IcpState* state, cudaStream_t s, bool inputs_ready) {
+                      int has_color, const IcpState* state, cudaStream_t s) {
   prepare_blocks(p, width, height, s);
   const kf_integration_options& o = p.config.integration;
   const uint32_t blocks = p.view.bx * p.view.by * p.view.bz;
@@ -992,7 +1047,6 @@ void launch_integrate(Pipeline& p, const float4* table, uint32_t width, uint32_t
       check(cudaGetLastError(), "band_compact_kernel launch");
     }
   } else {
-    if (!inputs_ready) launch_integrate_inputs(p, table, width, height, s);
     const TileLevels lv = tile_levels_of(p);
     // block culling
     CullParams cp;
@@ -1067,24 +1121,66 @@ void launch_fill_volume(Pipeline& p, cudaStream_t s) {
   reset_blocks(p, s);
 }
 
+namespace {
+// The arguments of for_touched_bricks; false when nothing was ever fused.
+struct Touched {
+  const uint4* voxel_bits;
+  const unsigned long long* allocated;
+  unsigned long long slots;
+};
+bool touched_bricks(const Pipeline& p, Touched& t) {
+  t = Touched{reinterpret_cast<const uint4*>(p.voxel_bits.ptr), nullptr, p.brick_class.count};
+  if (p.view.table != nullptr) t = Touched{nullptr, p.allocated.ptr, p.sparse_capacity};
+  return t.allocated != nullptr || t.slots != 0;  // dense: the skip structures exist from the first integration on
+}
+}  // namespace
+
+void launch_refill_volume(Pipeline& p, cudaStream_t s) {
+  Touched t;
+  if (!touched_bricks(p, t)) return;
+  const unsigned grid = 148 * 8;
+  float4* colors = p.config.color == KF_COLOR_FLOAT ? p.colors.ptr : nullptr;
+  switch (p.config.voxel) {
+    case KF_VOXEL_QUANTIZED:
+      refill_kernel<KF_VOXEL_QUANTIZED><<<grid, 256, 0, s>>>(p.voxels.ptr, colors, t.voxel_bits, t.allocated, t.slots);
+      break;
+    case KF_VOXEL_BF16:
+      refill_kernel<KF_VOXEL_BF16><<<grid, 256, 0, s>>>(p.voxels.ptr, colors, t.voxel_bits, t.allocated, t.slots);
+      break;
+    default:
+      refill_kernel<KF_VOXEL_FLOAT><<<grid, 256, 0, s>>>(p.voxels.ptr, colors, t.voxel_bits, t.allocated, t.slots);
+      break;
+  }
+  check(cudaGetLastError(), "refill_kernel launch");
+}
+
 uint64_t count_observed(Pipeline& p) {
-  DeviceArray<unsigned long long> result(1);
-  check(cudaMemsetAsync(result.ptr, 0, sizeof(unsigned long long), p.stream), "count clear");
+  Touched t;
+  if (!touched_bricks(p, t)) {
+    check(cudaStreamSynchronize(p.stream), "count observed");
+    return 0;
+  }
+  p.observed_count.resize(1);
+  check(cudaMemsetAsync(p.observed_count.ptr, 0, sizeof(unsigned long long), p.stream), "count clear");
   const unsigned grid = 148 * 8;
   switch (p.config.voxel) {
     case KF_VOXEL_QUANTIZED:
-      count_observed_kernel<KF_VOXEL_QUANTIZED><<<grid, 256, 0, p.stream>>>(p.voxels.ptr, p.voxel_count, result.ptr);
+      count_observed_kernel<KF_VOXEL_QUANTIZED>
+          <<<grid, 256, 0, p.stream>>>(p.voxels.ptr, t.voxel_bits, t.allocated, t.slots, p.observed_count.ptr);
       break;
     case KF_VOXEL_BF16:
-      count_observed_kernel<KF_VOXEL_BF16><<<grid, 256, 0, p.stream>>>(p.voxels.ptr, p.voxel_count, result.ptr);
+      count_observed_kernel<KF_VOXEL_BF16>
+          <<<grid, 256, 0, p.stream>>>(p.voxels.ptr, t.voxel_bits, t.allocated, t.slots, p.observed_count.ptr);
       break;
     default:
-      count_observed_kernel<KF_VOXEL_FLOAT><<<grid, 256, 0, p.stream>>>(p.voxels.ptr, p.voxel_count, result.ptr);
+      count_observed_kernel<KF_VOXEL_FLOAT>
+          <<<grid, 256, 0, p.stream>>>(p.voxels.ptr, t.voxel_bits, t.allocated, t.slots, p.observed_count.ptr);
       break;
   }
   check(cudaGetLastError(), "count_observed_kernel launch");
   unsigned long long host = 0;
-  check(cudaMemcpyAsync(&host, result.ptr, sizeof(host), cudaMemcpyDeviceToHost, p.stream), "count download");
+  check(cudaMemcpyAsync(&host, p.observed_count.ptr, sizeof(host), cudaMemcpyDeviceToHost, p.stream),
+        "count download");
   check(cudaStreamSynchronize(p.stream), "count observed");
   return host;
 }

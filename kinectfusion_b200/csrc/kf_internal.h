@@ -354,6 +354,7 @@ struct Pipeline {
   };
   std::map<std::pair<uint32_t, uint32_t>, Maps> maps;
   cudaStream_t stream = nullptr;
+  DeviceArray<unsigned long long> observed_count;  // kf_pipeline_observed_voxel_count's result
   DeviceArray<unsigned long long> counters;  // [0] voxel updates, [1] colour updates
   cudaEvent_t kernel_start = nullptr, kernel_stop = nullptr;  // borrowed
   // whole-frame graphs keyed by (width, height, iterations, first, colour, fork)
@@ -420,20 +421,16 @@ inline uint32_t null_cells_along(uint32_t blocks, int level) {
 
 // Integration pixel table: depth meters (NaN if unusable), lambda, fusion
 // weight and colour, one float4 per pixel.
-void launch_pixel_table(const uint16_t* depth, const uint32_t* color, const float* normals,
-                        uint32_t width, uint32_t height, Intr intrinsics,
-                        const kf_integration_options& options, int rule, float4* table,
-                        cudaStream_t stream);
+// For the full sweep also the depth-tile pyramid of its block culling.  Needs
+// the frame only, not the pose.
+void launch_pixel_table(Pipeline& p, const uint16_t* depth, const uint32_t* color, const float* normals,
+                        uint32_t width, uint32_t height, Intr intrinsics, float4* table, cudaStream_t stream);
 // Dense full sweep.  `pose_state` (optional) overrides world_to_camera with
 // the inverse of the tracked pose and skips fusion when tracking failed.
-// With `inputs_ready` the steps of launch_integrate_inputs already ran.
+// Follows launch_pixel_table of the same frame.
 void launch_integrate(Pipeline& p, const float4* table, uint32_t width, uint32_t height,
                       Intr intrinsics, Rigid world_to_camera, int has_color,
-                      const IcpState* pose_state, cudaStream_t stream, bool inputs_ready = false);
-// The integration steps that need only the frame's pixel table, not the pose:
-// the depth-tile pyramid of the full sweep's block culling.
-void launch_integrate_inputs(Pipeline& p, const float4* table, uint32_t width, uint32_t height,
-                             cudaStream_t stream);
+                      const IcpState* pose_state, cudaStream_t stream);
 // Allocates and clears the per-block skip and culling buffers.
 // C = A * B^T (+bias)(ReLU) on the tensor cores: A M x K, B N x K bf16
 // row-major (leading dimensions lda, ldb), C M x N fp32 (ldc).  `error`
@@ -455,7 +452,11 @@ void launch_band_rebuild(Pipeline& p, cudaStream_t stream);
 void launch_raycast(const Pipeline& p, const kf_raycast_camera& camera, float* points,
                     float* normals, uint32_t* colors, const IcpState* pose_state,
                     cudaStream_t stream);
+// A new volume: every voxel unobserved.
 void launch_fill_volume(Pipeline& p, cudaStream_t stream);
+// The same after use: the bricks that integrations wrote.  Before the skip
+// structures and the sparse counters are reset.
+void launch_refill_volume(Pipeline& p, cudaStream_t stream);
 uint64_t count_observed(Pipeline& p);
 // Sparse storage: every block unallocated again.
 void reset_sparse(Pipeline& p, cudaStream_t stream);
