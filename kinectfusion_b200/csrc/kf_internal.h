@@ -354,6 +354,9 @@ struct Pipeline {
   };
   std::map<std::pair<uint32_t, uint32_t>, Maps> maps;
   cudaStream_t stream = nullptr;
+  // kf_pipeline_extract_mesh's working arrays and page-locked staging
+  DeviceArray<uint8_t> mesh_cells, mesh_surface;
+  PinnedArray<uint8_t> mesh_staging;
   DeviceArray<unsigned long long> observed_count;  // kf_pipeline_observed_voxel_count's result
   DeviceArray<unsigned long long> counters;  // [0] voxel updates, [1] colour updates
   cudaEvent_t kernel_start = nullptr, kernel_stop = nullptr;  // borrowed

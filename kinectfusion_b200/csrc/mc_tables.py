@@ -165,19 +165,23 @@ def main():
         "",
         "#include <stdint.h>",
         "",
-        "static const uint8_t kMcCorner[8][3] = {" + ", ".join("{%d, %d, %d}" % c for c in CORNERS) + "};",
+        "#ifndef KF_MC_TABLE",
+        "#define KF_MC_TABLE static const",
+        "#endif",
+        "",
+        "KF_MC_TABLE uint8_t kMcCorner[8][3] = {" + ", ".join("{%d, %d, %d}" % c for c in CORNERS) + "};",
     ]
     axes = []
     for p, q in EDGES:
         d = [CORNERS[q][i] - CORNERS[p][i] for i in range(3)]
         axes.append(d.index(1))
-    lines.append("static const uint8_t kMcEdge[12][3] = {" +
+    lines.append("KF_MC_TABLE uint8_t kMcEdge[12][3] = {" +
                  ", ".join("{%d, %d, %d}" % (p, q, a) for (p, q), a in zip(EDGES, axes)) + "};")
-    lines.append("static const uint16_t kMcEdgeMask[256] = {")
+    lines.append("KF_MC_TABLE uint16_t kMcEdgeMask[256] = {")
     for i in range(0, 256, 16):
         lines.append("    " + ", ".join("0x%03x" % m for m in masks[i:i + 16]) + ",")
     lines.append("};")
-    lines.append("static const int8_t kMcTriangles[256][16] = {")
+    lines.append("KF_MC_TABLE int8_t kMcTriangles[256][16] = {")
     for row in table:
         lines.append("    {" + ", ".join("%d" % v for v in row) + "},")
     lines.append("};")
