@@ -102,7 +102,7 @@ template <int BN>
 __global__ void __launch_bounds__(kGemmThreads)
     gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                      float* __restrict__ C, int M, int N, int K, int ldc, const float* __restrict__ bias, int relu,
-                     int slabs, int gm, int gn, int* __restrict__ error) {
+                     int slabs, int gm, int gn, int* __restrict__ error, __nv_bfloat16* __restrict__ out_bf16) {
   constexpr uint32_t kCols = BN < 32 ? 32 : BN;  // tensor-memory columns (a power of two >= 32)
   constexpr uint32_t kStageA = kGemmBM * kGemmBK * 2, kStageB = BN * kGemmBK * 2;
   constexpr uint32_t kStageBytes = kStageA + kStageB;  // a multiple of 1024 for every BN
@@ -204,30 +204,52 @@ __global__ void __launch_bounds__(kGemmThreads)
     asm volatile("tcgen05.fence::after_thread_sync;");
     const bool split = gridDim.z > 1;
     float* out = C + (split ? static_cast<size_t>(blockIdx.z) * M * ldc : 0u);
-    const int row = tile_m + warp * 32 + lane;
-#pragma unroll
-    for (int c = 0; c < BN; c += 16) {
-      uint32_t r[16];
+    // Tensor memory hands each thread a row; the warp turns 32 x 32 values at
+    // a time in shared memory (the stages are free now) and stores rows, so a
+    // store fills whole lines instead of a word in each of 32 (19200 x 288 x 32:
+    // 20.8 us against 70 us).
+    float* turn = reinterpret_cast<float*>(base) + warp * (32 * 33);
+    const int first_row = tile_m + warp * 32;
+#pragma unroll 1
+    for (int c = 0; c < BN; c += 32) {
+      if (tile_n + c >= N || first_row >= M) break;  // the same for every lane
+      uint32_t r[32];
       const uint32_t addr = tmem + (static_cast<uint32_t>(warp * 32) << 16) + static_cast<uint32_t>(c);
       asm volatile(
-          "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+          "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,"
+          "%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
           : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-            "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+            "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
+            "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
+            "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
           : "r"(addr));
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-      if (row < M) {
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          const int col = tile_n + c + j;
-          if (col >= N) continue;
-          float v = nslabs > 0 ? __uint_as_float(r[j]) : 0.0f;
-          if (!split) {
-            if (bias != nullptr) v += bias[col];
-            if (relu && v < 0.0f) v = 0.0f;
-          }
-          out[static_cast<size_t>(row) * ldc + col] = v;
+      for (int j = 0; j < 32; ++j) turn[lane * 33 + j] = nslabs > 0 ? __uint_as_float(r[j]) : 0.0f;
+      __syncwarp();
+      const int col = tile_n + c + lane;
+      const bool in_tile = col < N && c + lane < BN;
+      const float add = !split && bias != nullptr && in_tile ? bias[col] : 0.0f;
+      auto store = [&](int i) {
+        float v = turn[i * 33 + lane];
+        if (!split) {
+          if (bias != nullptr) v += add;
+          if (relu && v < 0.0f) v = 0.0f;
+        }
+        const size_t at = static_cast<size_t>(first_row + i) * ldc + col;
+        out[at] = v;
+        if (!split && out_bf16 != nullptr) out_bf16[at] = __float2bfloat16(v);
+      };
+      if (in_tile) {
+        const int n = min(32, M - first_row);
+        if (n == 32) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) store(i);
+        } else {
+          for (int i = 0; i < n; ++i) store(i);
         }
       }
+      __syncwarp();
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;");
@@ -237,15 +259,28 @@ __global__ void __launch_bounds__(kGemmThreads)
 
 // C = sum over the split partials (in split order) (+ bias) (ReLU).
 __global__ void gemm_splitk_reduce_kernel(const float* __restrict__ partial, int splits, int M, int N, int ldp,
-                                          float* __restrict__ C, int ldc, const float* __restrict__ bias, int relu) {
+                                          float* __restrict__ C, int ldc, const float* __restrict__ bias, int relu,
+                                          __nv_bfloat16* __restrict__ out_bf16) {
   const size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= static_cast<size_t>(M) * N) return;
   const int row = static_cast<int>(i / N), col = static_cast<int>(i % N);
   float v = 0.0f;
-  for (int z = 0; z < splits; ++z) v += partial[(static_cast<size_t>(z) * M + row) * ldp + col];
+  // sixteen loads in flight, added in split order
+  const float* in = partial + static_cast<size_t>(row) * ldp + col;
+  const size_t step = static_cast<size_t>(M) * ldp;
+  int z = 0;
+  for (; z + 16 <= splits; z += 16) {
+    float x[16];
+#pragma unroll
+    for (int u = 0; u < 16; ++u) x[u] = in[(z + u) * step];
+#pragma unroll
+    for (int u = 0; u < 16; ++u) v += x[u];
+  }
+  for (; z < splits; ++z) v += in[z * step];
   if (bias != nullptr) v += bias[col];
   if (relu && v < 0.0f) v = 0.0f;
   C[static_cast<size_t>(row) * ldc + col] = v;
+  if (out_bf16 != nullptr) out_bf16[static_cast<size_t>(row) * ldc + col] = __float2bfloat16(v);
 }
 
 using EncodeTiled = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -280,7 +315,8 @@ CUtensorMap tensor_map(const void* base, int rows, int K, int ld, int box_rows) 
 
 template <int BN>
 void launch_tiles(const __nv_bfloat16* a, const __nv_bfloat16* b, float* c, int M, int N, int K, int lda, int ldb,
-                  int ldc, const float* bias, int relu, int slabs, unsigned splits, int* error, cudaStream_t s) {
+                  int ldc, const float* bias, int relu, int slabs, unsigned splits, int* error, __nv_bfloat16* out_bf16,
+                  cudaStream_t s) {
   static bool configured = false;  // per process: every device gets the same attribute
   if (!configured) {
     check(cudaFuncSetAttribute(gemm_bf16_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -293,14 +329,15 @@ void launch_tiles(const __nv_bfloat16* a, const __nv_bfloat16* b, float* c, int 
   const unsigned gm = ceil_div(static_cast<unsigned>(M), static_cast<unsigned>(kGemmBM));
   const unsigned gn = ceil_div(static_cast<unsigned>(N), static_cast<unsigned>(BN));
   gemm_bf16_kernel<BN><<<dim3(gm * gn, 1, splits), kGemmThreads, gemm_smem_bytes<BN>(), s>>>(
-      ma, mb, c, M, N, K, ldc, bias, relu, slabs, static_cast<int>(gm), static_cast<int>(gn), error);
+      ma, mb, c, M, N, K, ldc, bias, relu, slabs, static_cast<int>(gm), static_cast<int>(gn), error, out_bf16);
 }
 
 }  // namespace
 
 void launch_gemm_bf16(const void* A, const void* B, float* C, int M, int N, int K, int lda, int ldb, int ldc,
                       const float* bias, int relu, int* error, cudaStream_t s, float* workspace,
-                      size_t workspace_floats) {
+                      size_t workspace_floats, void* C_bf16) {
+  auto* out_bf16 = static_cast<__nv_bfloat16*>(C_bf16);
   require(M > 0 && N > 0 && K > 0, "gemm: empty shape");
   require(lda % 8 == 0 && ldb % 8 == 0 && K % 8 == 0, "gemm: K and the leading dimensions must be multiples of 8");
   require(reinterpret_cast<uintptr_t>(A) % 16 == 0 && reinterpret_cast<uintptr_t>(B) % 16 == 0,
@@ -327,17 +364,17 @@ void launch_gemm_bf16(const void* A, const void* B, float* C, int M, int N, int 
   float* out = splits > 1 ? workspace : C;
   const int ldo = splits > 1 ? N : ldc;
   switch (bn) {
-    case 16: launch_tiles<16>(a, b, out, M, N, K, lda, ldb, ldo, bias, relu, slabs, splits, error, s); break;
-    case 32: launch_tiles<32>(a, b, out, M, N, K, lda, ldb, ldo, bias, relu, slabs, splits, error, s); break;
-    case 64: launch_tiles<64>(a, b, out, M, N, K, lda, ldb, ldo, bias, relu, slabs, splits, error, s); break;
-    case 128: launch_tiles<128>(a, b, out, M, N, K, lda, ldb, ldo, bias, relu, slabs, splits, error, s); break;
-    default: launch_tiles<256>(a, b, out, M, N, K, lda, ldb, ldo, bias, relu, slabs, splits, error, s); break;
+    case 16: launch_tiles<16>(a, b, out, M, N, K, lda, ldb, ldo, bias, relu, slabs, splits, error, out_bf16, s); break;
+    case 32: launch_tiles<32>(a, b, out, M, N, K, lda, ldb, ldo, bias, relu, slabs, splits, error, out_bf16, s); break;
+    case 64: launch_tiles<64>(a, b, out, M, N, K, lda, ldb, ldo, bias, relu, slabs, splits, error, out_bf16, s); break;
+    case 128: launch_tiles<128>(a, b, out, M, N, K, lda, ldb, ldo, bias, relu, slabs, splits, error, out_bf16, s); break;
+    default: launch_tiles<256>(a, b, out, M, N, K, lda, ldb, ldo, bias, relu, slabs, splits, error, out_bf16, s); break;
   }
   check(cudaGetLastError(), "gemm_bf16_kernel launch");
   if (splits > 1) {
     const size_t n = static_cast<size_t>(M) * N;
     gemm_splitk_reduce_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, s>>>(workspace, static_cast<int>(splits),
-                                                                                  M, N, N, C, ldc, bias, relu);
+                                                                                  M, N, N, C, ldc, bias, relu, out_bf16);
     check(cudaGetLastError(), "gemm_splitk_reduce_kernel launch");
   }
 }

@@ -64,51 +64,58 @@ unsigned blocks_for(size_t n) { return static_cast<unsigned>((n + 255) / 256); }
 
 // ---- small kernels ----------------------------------------------------------
 // im2col of an NHWC bf16 map: row (b, oy, ox), column c*9 + ky*3 + kx (zero
-// outside the image and in the columns past k).
-__global__ void im2col_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ col, int batch,
-                              Conv c) {
-  const size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  const size_t total = static_cast<size_t>(batch) * c.hout * c.wout * c.kpad;
-  if (i >= total) return;
-  const int kk = static_cast<int>(i % c.kpad);
-  const size_t row = i / c.kpad;
-  const int ox = static_cast<int>(row % c.wout), oy = static_cast<int>((row / c.wout) % c.hout);
-  const int b = static_cast<int>(row / (static_cast<size_t>(c.wout) * c.hout));
-  __nv_bfloat16 v = __float2bfloat16(0.0f);
-  if (kk < c.k) {
-    const int ch = kk / 9, ky = (kk / 3) % 3, kx = kk % 3;
+// outside the image and in the columns past k).  A thread writes eight columns
+// with one 16-byte store; the layer's shape is a constant, so its index
+// arithmetic has no divisions (batch 64: 14.7, 38.9, 12.7 and 7.5 us with a
+// thread per element and the shape as an argument; 7.0, 13.0,
+// 5.7 and 4.6 us).
+template <int L>
+__global__ void __launch_bounds__(256)
+    im2col_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ col, int batch) {
+  constexpr Conv c = kConv[L];
+  static_assert(c.kpad % 8 == 0, "whole 16-byte stores");
+  const int i = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x);
+  if (i >= batch * (c.hout * c.wout * (c.kpad / 8))) return;
+  const int k0 = i % (c.kpad / 8) * 8, row = i / (c.kpad / 8);
+  const int ox = row % c.wout, oy = (row / c.wout) % c.hout, b = row / (c.wout * c.hout);
+  const unsigned short* in = reinterpret_cast<const unsigned short*>(x) + b * (c.hin * c.win * c.cin);
+  unsigned short v[8];
+#pragma unroll
+  for (int u = 0; u < 8; ++u) {
+    const int kk = k0 + u, ch = kk / 9, ky = (kk / 3) % 3, kx = kk % 3;
     const int y = oy * 2 - 1 + ky, xx = ox * 2 - 1 + kx;
-    if (y >= 0 && y < c.hin && xx >= 0 && xx < c.win) {
-      v = x[((static_cast<size_t>(b) * c.hin + y) * c.win + xx) * c.cin + ch];
-    }
+    v[u] = kk < c.k && y >= 0 && y < c.hin && xx >= 0 && xx < c.win ? __ldg(in + (y * c.win + xx) * c.cin + ch) : 0;
   }
-  col[i] = v;
+  uint4 w;
+  w.x = v[0] | (static_cast<uint32_t>(v[1]) << 16);
+  w.y = v[2] | (static_cast<uint32_t>(v[3]) << 16);
+  w.z = v[4] | (static_cast<uint32_t>(v[5]) << 16);
+  w.w = v[6] | (static_cast<uint32_t>(v[7]) << 16);
+  reinterpret_cast<uint4*>(col)[i] = w;
 }
 
 // col2im in gather form (one thread per input element, fixed order): dx = the
 // sum of dcol over the output positions whose 3x3 window holds the element.
-__global__ void col2im_kernel(const float* __restrict__ dcol, float* __restrict__ dx, int batch, Conv c) {
-  const size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  const size_t total = static_cast<size_t>(batch) * c.hin * c.win * c.cin;
-  if (i >= total) return;
-  const int ch = static_cast<int>(i % c.cin);
-  const size_t p = i / c.cin;
-  const int x = static_cast<int>(p % c.win), y = static_cast<int>((p / c.win) % c.hin);
-  const int b = static_cast<int>(p / (static_cast<size_t>(c.win) * c.hin));
-  float s = 0.0f;
-  for (int ky = 0; ky < 3; ++ky) {
-    const int ty = y + 1 - ky;
-    if (ty < 0 || (ty & 1)) continue;
-    const int oy = ty / 2;
-    if (oy >= c.hout) continue;
-    for (int kx = 0; kx < 3; ++kx) {
-      const int tx = x + 1 - kx;
-      if (tx < 0 || (tx & 1)) continue;
-      const int ox = tx / 2;
-      if (ox >= c.wout) continue;
-      s += dcol[((static_cast<size_t>(b) * c.hout + oy) * c.wout + ox) * c.kpad + ch * 9 + ky * 3 + kx];
-    }
+template <int L>
+__global__ void __launch_bounds__(256)
+    col2im_kernel(const float* __restrict__ dcol, float* __restrict__ dx, int batch) {
+  constexpr Conv c = kConv[L];
+  const int i = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x);
+  if (i >= batch * (c.hin * c.win * c.cin)) return;
+  const int ch = i % c.cin, p = i / c.cin;
+  const int x = p % c.win, y = (p / c.win) % c.hin, b = p / (c.win * c.hin);
+  // at most two window rows and columns reach the element: their loads are
+  // issued together, then added in the windows' order
+  float v[9];
+#pragma unroll
+  for (int k = 0; k < 9; ++k) {
+    const int ty = y + 1 - k / 3, tx = x + 1 - k % 3, oy = ty >> 1, ox = tx >> 1;
+    const bool in = ty >= 0 && tx >= 0 && ((ty | tx) & 1) == 0 && oy < c.hout && ox < c.wout;
+    v[k] = in ? __ldg(dcol + ((b * c.hout + oy) * c.wout + ox) * c.kpad + ch * 9 + k) : 0.0f;
   }
+  float s = 0.0f;
+#pragma unroll
+  for (int k = 0; k < 9; ++k) s += v[k];
   dx[i] = s;
 }
 
@@ -117,43 +124,82 @@ __global__ void to_bf16_kernel(const float* __restrict__ in, __nv_bfloat16* __re
   if (i < n) out[i] = __float2bfloat16(in[i]);
 }
 
-// out[c][r] = bf16(in[r][c]) for an R x C fp32 matrix (leading dimension
-// in_ld); rows r >= R of each output line (up to out_ld) are zero.
-__global__ void transpose_bf16_kernel(const float* __restrict__ in, int rows, int cols, int in_ld,
-                                      __nv_bfloat16* __restrict__ out, int out_ld) {
-  const size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= static_cast<size_t>(cols) * out_ld) return;
-  const int r = static_cast<int>(i % out_ld), c = static_cast<int>(i / out_ld);
-  out[i] = __float2bfloat16(r < rows ? in[static_cast<size_t>(r) * in_ld + c] : 0.0f);
+// out[c][r] = in[r][c] for an R x C bf16 matrix; rows r >= R of each output
+// line (up to out_ld) are zero.  32 x 32 tiles through shared memory, so both
+// sides move whole sectors (19200 x 288: 27.2 us with a strided read per
+// element, 15.4 us).
+__global__ void __launch_bounds__(256)
+    transpose_bf16_kernel(const unsigned short* __restrict__ in, int rows, int cols, unsigned short* __restrict__ out,
+                          int out_ld) {
+  __shared__ unsigned short s_tile[32][34];
+  const int r0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
+#pragma unroll
+  for (int j = threadIdx.y; j < 32; j += 8) {
+    const int r = r0 + j, c = c0 + threadIdx.x;
+    s_tile[j][threadIdx.x] = r < rows && c < cols ? in[static_cast<size_t>(r) * cols + c] : 0;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int j = threadIdx.y; j < 32; j += 8) {
+    const int c = c0 + j, r = r0 + threadIdx.x;
+    if (c < cols && r < out_ld) out[static_cast<size_t>(c) * out_ld + r] = s_tile[threadIdx.x][j];
+  }
 }
 
-// the same for a bf16 matrix
-__global__ void transpose_bf16_bf16_kernel(const __nv_bfloat16* __restrict__ in, int rows, int cols, int in_ld,
-                                           __nv_bfloat16* __restrict__ out, int out_ld) {
-  const size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= static_cast<size_t>(cols) * out_ld) return;
-  const int r = static_cast<int>(i % out_ld), c = static_cast<int>(i / out_ld);
-  out[i] = r < rows ? in[static_cast<size_t>(r) * in_ld + c] : __float2bfloat16(0.0f);
+// The bf16 transposed weights of all layers: out[c][r] = bf16(in[r][c]),
+// rows past R up to rows_pad zero.  One launch, a grid row per layer.
+struct WeightTransposes {
+  const float* in[6];
+  __nv_bfloat16* out[6];
+  int rows[6], cols[6], rows_pad[6];
+};
+__global__ void transpose_weights_kernel(WeightTransposes w) {
+  const int l = blockIdx.y, n = w.cols[l] * w.rows_pad[l];
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const int r = i % w.rows_pad[l], c = i / w.rows_pad[l];
+    w.out[l][i] = __float2bfloat16(r < w.rows[l] ? w.in[l][r * w.cols[l] + c] : 0.0f);
+  }
 }
 
-// dz = dy where the layer's ReLU output was positive, else 0 (in place)
-__global__ void relu_back_kernel(float* __restrict__ dy, const float* __restrict__ a, size_t n) {
-  const size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i < n && !(a[i] > 0.0f)) dy[i] = 0.0f;
-}
-
-// Column sums of an R x C fp32 matrix (bias gradients) in two fixed-order
-// stages: CTA (x, y) sums rows [256 y, 256 y + 256) of columns [32 x, 32 x +
-// 32) into partial[y][c]; colsum_finish adds the partials in order.
+// The gradient dy of a layer's output (R x C fp32), made ready for the GEMMs
+// and the bias sum in one pass: dz = dy where the ReLU output `a` was
+// positive, else 0 (a null: no ReLU), as bf16 rows (`rows_out`, or null) and
+// as bf16 columns (`cols_out`, leading dimension out_ld, zero past R), and the
+// column sums of dz over chunks of 256 rows, each in a fixed order, into
+// partial[chunk][c].  (Masking, rounding, transposing and summing in four
+// kernels took 44 us for conv1 at batch 64, 21.7 us.)
 constexpr int kColsumRows = 256;
-__global__ void colsum_partial_kernel(const float* __restrict__ m, int rows, int cols, float* __restrict__ partial) {
+__global__ void __launch_bounds__(256)
+    dz_kernel(const float* __restrict__ dy, const float* __restrict__ a, int rows, int cols,
+              __nv_bfloat16* __restrict__ rows_out, __nv_bfloat16* __restrict__ cols_out, int out_ld,
+              float* __restrict__ partial) {
   __shared__ float s[8][33];
+  __shared__ __align__(16) __nv_bfloat16 s_cols[32][kColsumRows + 2];  // 129 words a column: no bank conflicts
   const int c = blockIdx.x * 32 + threadIdx.x;
   const int r0 = blockIdx.y * kColsumRows;
   float acc = 0.0f;
-  if (c < cols) {
-    const int r1 = min(rows, r0 + kColsumRows);
-    for (int r = r0 + threadIdx.y; r < r1; r += 8) acc += m[static_cast<size_t>(r) * cols + c];
+#pragma unroll
+  for (int j0 = 0; j0 < kColsumRows / 8; j0 += 16) {
+    float v[16], act[16];
+#pragma unroll
+    for (int u = 0; u < 16; ++u) {
+      const int r = r0 + threadIdx.y + 8 * (j0 + u);
+      const bool in = r < rows && c < cols;
+      const size_t at = in ? static_cast<size_t>(r) * cols + c : 0;
+      v[u] = in ? __ldg(dy + at) : 0.0f;
+      act[u] = in && a != nullptr ? __ldg(a + at) : 1.0f;
+    }
+#pragma unroll
+    for (int u = 0; u < 16; ++u) {
+      const int in_chunk = threadIdx.y + 8 * (j0 + u), r = r0 + in_chunk;
+      const float dz = act[u] > 0.0f ? v[u] : 0.0f;
+      const __nv_bfloat16 b = __float2bfloat16(dz);
+      if (r < rows && c < cols) {
+        acc += dz;
+        if (rows_out != nullptr) rows_out[static_cast<size_t>(r) * cols + c] = b;
+      }
+      s_cols[threadIdx.x][in_chunk] = b;
+    }
   }
   s[threadIdx.y][threadIdx.x] = acc;
   __syncthreads();
@@ -162,13 +208,40 @@ __global__ void colsum_partial_kernel(const float* __restrict__ m, int rows, int
     for (int j = 0; j < 8; ++j) t += s[j][threadIdx.x];
     partial[static_cast<size_t>(blockIdx.y) * cols + c] = t;
   }
+  // eight rows of a column per lane: out_ld and r0 are multiples of 8
+  for (int j = threadIdx.y; j < 32; j += 8) {
+    const int oc = blockIdx.x * 32 + j, r = r0 + static_cast<int>(threadIdx.x) * 8;
+    if (oc < cols && r < out_ld) {
+      const uint32_t* w = reinterpret_cast<const uint32_t*>(&s_cols[j][threadIdx.x * 8]);
+      *reinterpret_cast<uint4*>(cols_out + static_cast<size_t>(oc) * out_ld + r) = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+  }
 }
-__global__ void colsum_finish_kernel(const float* __restrict__ partial, int chunks, int cols, float* __restrict__ out) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= cols) return;
+
+// Column sums from the chunks' partials, in chunk order: a CTA stages 32
+// columns, a thread adds each (300 chunks: 19.3 us straight from memory,
+// 9.3 us).
+constexpr int kFinishChunks = 128;
+__global__ void __launch_bounds__(256)
+    colsum_finish_kernel(const float* __restrict__ partial, int chunks, int cols, int keep, float* __restrict__ out) {
+  __shared__ float s_part[kFinishChunks][32];
+  const int lane = threadIdx.x & 31, c = blockIdx.x * 32 + lane;
   float t = 0.0f;
-  for (int j = 0; j < chunks; ++j) t += partial[static_cast<size_t>(j) * cols + c];
-  out[c] = t;
+  for (int j0 = 0; j0 < chunks; j0 += kFinishChunks) {
+    const int n = min(kFinishChunks, chunks - j0);
+#pragma unroll
+    for (int u = 0; u < kFinishChunks / 8; ++u) {
+      const int j = static_cast<int>(threadIdx.x >> 5) + 8 * u;
+      if (j < n && c < cols) s_part[j][lane] = __ldg(partial + static_cast<size_t>(j0 + j) * cols + c);
+    }
+    __syncthreads();
+    if (threadIdx.x < 32 && c < keep) {
+#pragma unroll 8
+      for (int j = 0; j < n; ++j) t += s_part[j][lane];
+    }
+    __syncthreads();
+  }
+  if (threadIdx.x < 32 && c < keep) out[c] = t;
 }
 
 // d_out = 2 (out - target) / B into a B x 8 matrix (columns 6, 7 zero); the
@@ -196,11 +269,11 @@ __global__ void loss_kernel(const float* __restrict__ out, const float* __restri
   if (threadIdx.x == 0) loss[0] = s_sum[0] / static_cast<float>(batch);
 }
 
-// Adam (Kingma & Ba 2015) on the flat parameter vector; c1, c2 are the bias
-// corrections 1 - beta^t.
+// Adam (Kingma & Ba 2015) on the flat parameter vector, and its bf16 copy;
+// c1, c2 are the bias corrections 1 - beta^t.
 __global__ void adam_kernel(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
-                            float* __restrict__ v, size_t n, float lr, float b1, float b2, float eps, float c1,
-                            float c2) {
+                            float* __restrict__ v, __nv_bfloat16* __restrict__ p_bf16, size_t n, float lr, float b1,
+                            float b2, float eps, float c1, float c2) {
   const size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float gi = g[i];
@@ -208,7 +281,9 @@ __global__ void adam_kernel(float* __restrict__ p, const float* __restrict__ g, 
   const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
   m[i] = mi;
   v[i] = vi;
-  p[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+  const float next = p[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+  p[i] = next;
+  p_bf16[i] = __float2bfloat16(next);
 }
 
 }  // namespace
@@ -222,7 +297,7 @@ struct Learner {
   DeviceArray<__nv_bfloat16> wtbf;  // bf16 transposed weights [cols][rows_pad] (the input-gradient GEMMs' B)
   size_t wt_off[6] = {};
   int rows_pad[6] = {};
-  DeviceArray<__nv_bfloat16> col[4], xbf[6], t_a, t_b;
+  DeviceArray<__nv_bfloat16> col[4], xbf[6], t_a, t_b, dz_rows;
   DeviceArray<float> act[5], dact[5], dcol, dout8, loss, out, partial;
   DeviceArray<float> workspace;  // split-K partials of the weight-gradient GEMMs
   DeviceArray<int> error;
@@ -260,6 +335,7 @@ struct Learner {
     check(cudaMemcpy(params.ptr, h.data(), h.size() * sizeof(float), cudaMemcpyHostToDevice), "learner init");
     check(cudaMemset(adam_m.ptr, 0, adam_m.bytes()), "learner init");
     check(cudaMemset(adam_v.ptr, 0, adam_v.bytes()), "learner init");
+    size_t dz_max = static_cast<size_t>(batch) * kHidden;
     size_t dcol_max = static_cast<size_t>(batch) * kFlat, t_max = static_cast<size_t>(batch) * kFlat;
     for (int i = 0; i < 4; ++i) {
       const Conv& c = kConv[i];
@@ -270,6 +346,7 @@ struct Learner {
       xbf[i].resize(static_cast<size_t>(batch) * c.hin * c.win * c.cin);
       dcol_max = std::max(dcol_max, rows * c.kpad);
       t_max = std::max(t_max, rows * std::max(c.kpad, c.cout));
+      dz_max = std::max(dz_max, rows * c.cout);
     }
     xbf[4].resize(static_cast<size_t>(batch) * kFlat);
     xbf[5].resize(static_cast<size_t>(batch) * kHidden);
@@ -278,6 +355,7 @@ struct Learner {
     dcol.resize(dcol_max);
     t_a.resize(t_max);
     t_b.resize(t_max);
+    dz_rows.resize(dz_max);
     dout8.resize(static_cast<size_t>(batch) * kOutPad);
     partial.resize(static_cast<size_t>((batch * kConv[0].hout * kConv[0].wout + kColsumRows - 1) / kColsumRows) *
                    kHidden);
@@ -290,25 +368,37 @@ struct Learner {
     check(cudaDeviceSynchronize(), "learner init");
   }
 
-  // the bf16 copies of the weights and of their transposes
-  void refresh_weights(cudaStream_t s) {
-    to_bf16_kernel<<<blocks_for(lay.total), 256, 0, s>>>(params.ptr, wbf.ptr, lay.total);
+  // the bf16 copies of the weights' transposes
+  void refresh_transposes(cudaStream_t s) {
+    WeightTransposes w;
     for (int i = 0; i < 6; ++i) {
-      transpose_bf16_kernel<<<blocks_for(static_cast<size_t>(lay.cols[i]) * rows_pad[i]), 256, 0, s>>>(
-          params.ptr + lay.w[i], lay.rows[i], lay.cols[i], lay.cols[i], wtbf.ptr + wt_off[i], rows_pad[i]);
+      w.in[i] = params.ptr + lay.w[i];
+      w.out[i] = wtbf.ptr + wt_off[i];
+      w.rows[i] = lay.rows[i];
+      w.cols[i] = lay.cols[i];
+      w.rows_pad[i] = rows_pad[i];
     }
+    transpose_weights_kernel<<<dim3(148, 6), 256, 0, s>>>(w);
     check(cudaGetLastError(), "learner weights");
   }
 
-  void gemm(const __nv_bfloat16* a, const __nv_bfloat16* b, float* c, int m, int n, int k, int lda, int ldb,
-            int ldc, const float* bias, int relu, cudaStream_t s) {
-    launch_gemm_bf16(a, b, c, m, n, k, lda, ldb, ldc, bias, relu, error.ptr, s, workspace.ptr, workspace.count);
+  // the bf16 copies of the weights and of their transposes
+  void refresh_weights(cudaStream_t s) {
+    to_bf16_kernel<<<blocks_for(lay.total), 256, 0, s>>>(params.ptr, wbf.ptr, lay.total);
+    refresh_transposes(s);
   }
 
-  void colsum(const float* m, int rows, int cols, float* sums, cudaStream_t s) {
-    const int chunks = (rows + kColsumRows - 1) / kColsumRows;
-    colsum_partial_kernel<<<dim3((cols + 31) / 32, chunks), dim3(32, 8), 0, s>>>(m, rows, cols, partial.ptr);
-    colsum_finish_kernel<<<(cols + 63) / 64, 64, 0, s>>>(partial.ptr, chunks, cols, sums);
+  void gemm(const __nv_bfloat16* a, const __nv_bfloat16* b, float* c, int m, int n, int k, int lda, int ldb,
+            int ldc, const float* bias, int relu, cudaStream_t s, __nv_bfloat16* c_bf16 = nullptr) {
+    launch_gemm_bf16(a, b, c, m, n, k, lda, ldb, ldc, bias, relu, error.ptr, s, workspace.ptr, workspace.count,
+                     c_bf16);
+  }
+
+  template <int L>
+  void im2col(const __nv_bfloat16* x, int batch, cudaStream_t s) {
+    constexpr Conv c = kConv[L];
+    im2col_kernel<L><<<blocks_for(static_cast<size_t>(batch) * c.hout * c.wout * (c.kpad / 8)), 256, 0, s>>>(
+        x, col[L].ptr, batch);
   }
 
   // inputs: bf16 NHWC [batch][60][80][2] -> out [batch][6]
@@ -317,69 +407,71 @@ struct Learner {
     for (int i = 0; i < 4; ++i) {
       const Conv& c = kConv[i];
       const size_t rows = static_cast<size_t>(batch) * c.hout * c.wout;
-      im2col_kernel<<<blocks_for(rows * c.kpad), 256, 0, s>>>(x, col[i].ptr, batch, c);
+      switch (i) {
+        case 0: im2col<0>(x, batch, s); break;
+        case 1: im2col<1>(x, batch, s); break;
+        case 2: im2col<2>(x, batch, s); break;
+        default: im2col<3>(x, batch, s); break;
+      }
+      __nv_bfloat16* next = xbf[i + 1].ptr;
       gemm(col[i].ptr, wbf.ptr + lay.w[i], act[i].ptr, static_cast<int>(rows), c.cout, c.kpad, c.kpad, c.kpad,
-           c.cout, params.ptr + lay.b[i], 1, s);
-      __nv_bfloat16* next = i < 3 ? xbf[i + 1].ptr : xbf[4].ptr;
-      to_bf16_kernel<<<blocks_for(rows * c.cout), 256, 0, s>>>(act[i].ptr, next, rows * c.cout);
+           c.cout, params.ptr + lay.b[i], 1, s, next);
       x = next;
     }
     gemm(xbf[4].ptr, wbf.ptr + lay.w[4], act[4].ptr, batch, kHidden, kFlat, kFlat, kFlat, kHidden,
-         params.ptr + lay.b[4], 1, s);
-    to_bf16_kernel<<<blocks_for(static_cast<size_t>(batch) * kHidden), 256, 0, s>>>(
-        act[4].ptr, xbf[5].ptr, static_cast<size_t>(batch) * kHidden);
+         params.ptr + lay.b[4], 1, s, xbf[5].ptr);
     gemm(xbf[5].ptr, wbf.ptr + lay.w[5], out.ptr, batch, kOut, kHidden, kHidden, kHidden, kOut,
          params.ptr + lay.b[5], 0, s);
     check(cudaGetLastError(), "learner forward");
   }
 
-  // dW [n_out][k] = bf16(dz)^T . in for dz [m][n_out] fp32 and in [m][k] bf16:
-  // C = A B^T with A = dz^T [n_out][m], B = in^T [k][m].
-  void weight_grad(const float* dz, int m, int n_out, const __nv_bfloat16* in, int k, float* dw, cudaStream_t s) {
+  // From dy [m][n] (the gradient of a layer's ReLU output `a`, or of a layer
+  // without one) and the layer's input [m][k] bf16: dz as bf16 rows into
+  // dz_rows (with want_rows), db [keep of n] and dW [n][k] = bf16(dz)^T . in,
+  // the product of A = dz^T [n][m] and B = in^T [k][m].
+  void layer_grads(const float* dy, const float* a, int m, int n, const __nv_bfloat16* in, int k, bool want_rows,
+                   float* dw, float* db, int keep, cudaStream_t s) {
     const int mp = (m + 7) / 8 * 8;
-    transpose_bf16_kernel<<<blocks_for(static_cast<size_t>(n_out) * mp), 256, 0, s>>>(dz, m, n_out, n_out, t_a.ptr,
-                                                                                     mp);
-    transpose_bf16_bf16_kernel<<<blocks_for(static_cast<size_t>(k) * mp), 256, 0, s>>>(in, m, k, k, t_b.ptr, mp);
-    gemm(t_a.ptr, t_b.ptr, dw, n_out, k, mp, mp, mp, k, nullptr, 0, s);
+    const int chunks = (mp + kColsumRows - 1) / kColsumRows;
+    dz_kernel<<<dim3((n + 31) / 32, chunks), dim3(32, 8), 0, s>>>(dy, a, m, n, want_rows ? dz_rows.ptr : nullptr,
+                                                                  t_a.ptr, mp, partial.ptr);
+    colsum_finish_kernel<<<(n + 31) / 32, 256, 0, s>>>(partial.ptr, (m + kColsumRows - 1) / kColsumRows, n, keep, db);
+    transpose_bf16_kernel<<<dim3((mp + 31) / 32, (k + 31) / 32), dim3(32, 8), 0, s>>>(
+        reinterpret_cast<const unsigned short*>(in), m, k, reinterpret_cast<unsigned short*>(t_b.ptr), mp);
+    gemm(t_a.ptr, t_b.ptr, dw, n, k, mp, mp, mp, k, nullptr, 0, s);
   }
 
   // gradients of the batch-mean squared twist error into grads (after forward)
   void backward(const float* target, int batch, cudaStream_t s) {
     loss_kernel<<<1, 256, 0, s>>>(out.ptr, target, batch, dout8.ptr, loss.ptr);
     // fc2: dW = d_out^T x5 (the first 6 rows of an 8-row product), db, dx5 = d_out W
-    weight_grad(dout8.ptr, batch, kOutPad, xbf[5].ptr, kHidden, dcol.ptr, s);
+    layer_grads(dout8.ptr, nullptr, batch, kOutPad, xbf[5].ptr, kHidden, true, dcol.ptr, grads.ptr + lay.b[5], kOut,
+                s);
     check(cudaMemcpyAsync(grads.ptr + lay.w[5], dcol.ptr, sizeof(float) * kOut * kHidden, cudaMemcpyDeviceToDevice,
                           s),
           "learner grads");
-    colsum(dout8.ptr, batch, kOutPad, dcol.ptr, s);
-    check(cudaMemcpyAsync(grads.ptr + lay.b[5], dcol.ptr, sizeof(float) * kOut, cudaMemcpyDeviceToDevice, s),
-          "learner grads");
-    to_bf16_kernel<<<blocks_for(static_cast<size_t>(batch) * kOutPad), 256, 0, s>>>(
-        dout8.ptr, t_a.ptr, static_cast<size_t>(batch) * kOutPad);
-    gemm(t_a.ptr, wtbf.ptr + wt_off[5], dact[4].ptr, batch, kHidden, kOutPad, kOutPad, rows_pad[5], kHidden,
+    gemm(dz_rows.ptr, wtbf.ptr + wt_off[5], dact[4].ptr, batch, kHidden, kOutPad, kOutPad, rows_pad[5], kHidden,
          nullptr, 0, s);
     // fc1
-    relu_back_kernel<<<blocks_for(static_cast<size_t>(batch) * kHidden), 256, 0, s>>>(
-        dact[4].ptr, act[4].ptr, static_cast<size_t>(batch) * kHidden);
-    weight_grad(dact[4].ptr, batch, kHidden, xbf[4].ptr, kFlat, grads.ptr + lay.w[4], s);
-    colsum(dact[4].ptr, batch, kHidden, grads.ptr + lay.b[4], s);
-    to_bf16_kernel<<<blocks_for(static_cast<size_t>(batch) * kHidden), 256, 0, s>>>(
-        dact[4].ptr, t_a.ptr, static_cast<size_t>(batch) * kHidden);
+    layer_grads(dact[4].ptr, act[4].ptr, batch, kHidden, xbf[4].ptr, kFlat, true, grads.ptr + lay.w[4],
+                grads.ptr + lay.b[4], kHidden, s);
     // dx4 = the gradient of conv4's output, [batch*20][64] = [batch][1280]
-    gemm(t_a.ptr, wtbf.ptr + wt_off[4], dact[3].ptr, batch, kFlat, kHidden, kHidden, rows_pad[4], kFlat, nullptr, 0,
-         s);
+    gemm(dz_rows.ptr, wtbf.ptr + wt_off[4], dact[3].ptr, batch, kFlat, kHidden, kHidden, rows_pad[4], kFlat, nullptr,
+         0, s);
     for (int i = 3; i >= 0; --i) {
       const Conv& c = kConv[i];
       const size_t rows = static_cast<size_t>(batch) * c.hout * c.wout;
-      relu_back_kernel<<<blocks_for(rows * c.cout), 256, 0, s>>>(dact[i].ptr, act[i].ptr, rows * c.cout);
-      weight_grad(dact[i].ptr, static_cast<int>(rows), c.cout, col[i].ptr, c.kpad, grads.ptr + lay.w[i], s);
-      colsum(dact[i].ptr, static_cast<int>(rows), c.cout, grads.ptr + lay.b[i], s);
+      layer_grads(dact[i].ptr, act[i].ptr, static_cast<int>(rows), c.cout, col[i].ptr, c.kpad, i != 0,
+                  grads.ptr + lay.w[i], grads.ptr + lay.b[i], c.cout, s);
       if (i == 0) break;
-      to_bf16_kernel<<<blocks_for(rows * c.cout), 256, 0, s>>>(dact[i].ptr, t_a.ptr, rows * c.cout);
-      gemm(t_a.ptr, wtbf.ptr + wt_off[i], dcol.ptr, static_cast<int>(rows), c.kpad, c.cout, c.cout, rows_pad[i],
+      gemm(dz_rows.ptr, wtbf.ptr + wt_off[i], dcol.ptr, static_cast<int>(rows), c.kpad, c.cout, c.cout, rows_pad[i],
            c.kpad, nullptr, 0, s);
-      col2im_kernel<<<blocks_for(static_cast<size_t>(batch) * c.hin * c.win * c.cin), 256, 0, s>>>(
-          dcol.ptr, dact[i - 1].ptr, batch, c);
+      const unsigned ctas = blocks_for(static_cast<size_t>(batch) * c.hin * c.win * c.cin);
+      switch (i) {
+        case 1: col2im_kernel<1><<<ctas, 256, 0, s>>>(dcol.ptr, dact[0].ptr, batch); break;
+        case 2: col2im_kernel<2><<<ctas, 256, 0, s>>>(dcol.ptr, dact[1].ptr, batch); break;
+        default: col2im_kernel<3><<<ctas, 256, 0, s>>>(dcol.ptr, dact[2].ptr, batch); break;
+      }
     }
     check(cudaGetLastError(), "learner backward");
   }
@@ -389,9 +481,9 @@ struct Learner {
     const float b1 = 0.9f, b2 = 0.999f;
     const float c1 = 1.0f - std::pow(b1, static_cast<float>(steps));
     const float c2 = 1.0f - std::pow(b2, static_cast<float>(steps));
-    adam_kernel<<<blocks_for(lay.total), 256, 0, s>>>(params.ptr, grads.ptr, adam_m.ptr, adam_v.ptr, lay.total, lr,
-                                                      b1, b2, 1e-8f, c1, c2);
-    refresh_weights(s);
+    adam_kernel<<<blocks_for(lay.total), 256, 0, s>>>(params.ptr, grads.ptr, adam_m.ptr, adam_v.ptr, wbf.ptr,
+                                                      lay.total, lr, b1, b2, 1e-8f, c1, c2);
+    refresh_transposes(s);
   }
 
   void check_batch(uint32_t batch, const char* what) const {
