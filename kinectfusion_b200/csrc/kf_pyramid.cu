@@ -144,6 +144,87 @@ __global__ void __launch_bounds__(kTileX* kTileY)
   out[row * width + col] = result;
 }
 
+// The same filter at radius 2, the default.  A pair of pixels has one weight,
+// whichever of the two is the window's centre (the depth difference enters
+// squared), so the CTA computes each pair once, for the twelve neighbours
+// after a pixel in row order, and a pixel reads the other twelve from the
+// pixels before it: 15 exponentials per pixel with the tile's border instead
+// of 25.  640x480: 19.49 us against 24.7 us.
+constexpr int kPairRows = 16;              // pixel rows of a CTA's tile
+constexpr int kPairSpanX = kTileX + 4;     // with the border
+constexpr int kPairSpanY = kPairRows + 4;
+constexpr int kPairs = 12;
+constexpr int kPairFrom = (kPairRows + 2) * kPairSpanX;  // pixels whose later neighbours matter
+__host__ __device__ constexpr int pair_dy(int f) { return f < 2 ? 0 : (f < 7 ? 1 : 2); }
+__host__ __device__ constexpr int pair_dx(int f) { return f < 2 ? f + 1 : (f < 7 ? f - 4 : f - 9); }
+__global__ void __launch_bounds__(256)
+    bilateral_pairs_kernel(const uint16_t* __restrict__ in, uint16_t* __restrict__ out, int width, int height,
+                           DepthParams p) {
+  __shared__ float s_metres[kPairSpanY * kPairSpanX], s_raw[kPairSpanY * kPairSpanX];
+  __shared__ float s_weight[kPairs][kPairFrom];
+  __shared__ double s_exp2[kExpTable];
+  const int tid = threadIdx.x;
+  const int left = static_cast<int>(blockIdx.x) * kTileX - 2, top = static_cast<int>(blockIdx.y) * kPairRows - 2;
+  for (int i = tid; i < kPairSpanY * kPairSpanX; i += 256) {
+    const int x = left + i % kPairSpanX, y = top + i / kPairSpanX;
+    float m = kNaN, value = 0.0f;
+    if (x >= 0 && y >= 0 && x < width && y < height) {
+      const uint16_t raw = __ldg(in + y * width + x);
+      value = static_cast<float>(raw);
+      if (!depth_in_range(raw, p.depth_scale, p.min_depth, p.max_depth, m)) m = kNaN;
+    }
+    s_metres[i] = m;
+    s_raw[i] = value;
+  }
+  if (tid < kExpTable) s_exp2[tid] = exp2(static_cast<double>(tid) * (1.0 / kExpTable));
+  __syncthreads();
+  for (int i = tid; i < kPairFrom; i += 256) {
+    const int x = i % kPairSpanX;
+    const float here = s_metres[i];
+#pragma unroll
+    for (int f = 0; f < kPairs; ++f) {
+      const int tx = x + pair_dx(f);
+      float weight = 0.0f;  // of an unusable neighbour, and of one past the border (never read)
+      if (tx >= 0 && tx < kPairSpanX) {
+        const float dd = s_metres[i + pair_dy(f) * kPairSpanX + pair_dx(f)] - here;
+        const float d2 = static_cast<float>(pair_dx(f) * pair_dx(f) + pair_dy(f) * pair_dy(f));
+        const float arg = (d2 * p.spatial_scale) + (dd * dd * p.range_scale);
+        if (arg >= -104.0f) weight = gaussian(arg, s_exp2);  // below: rounds to zero
+      }
+      s_weight[f][i] = weight;
+    }
+  }
+  __syncthreads();
+  const int col = left + 2 + tid % kTileX;
+  for (int ty = tid / kTileX; ty < kPairRows; ty += 256 / kTileX) {
+    const int row = top + 2 + ty;
+    if (col >= width || row >= height) continue;
+    const int at = (ty + 2) * kPairSpanX + tid % kTileX + 2;
+    uint16_t result = 0;
+    if (s_metres[at] == s_metres[at]) {
+      float weighted_sum = 0.0f, weight_sum = 0.0f;
+      // the window in row order; a zero weight adds nothing, as skipping does
+#pragma unroll
+      for (int f = kPairs - 1; f >= 0; --f) {
+        const int from = at - pair_dy(f) * kPairSpanX - pair_dx(f);
+        const float weight = s_weight[f][from];
+        weighted_sum += weight * s_raw[from];
+        weight_sum += weight;
+      }
+      weighted_sum += s_raw[at];  // the centre's weight is exactly 1
+      weight_sum += 1.0f;
+#pragma unroll
+      for (int f = 0; f < kPairs; ++f) {
+        const float weight = s_weight[f][at];
+        weighted_sum += weight * s_raw[at + pair_dy(f) * kPairSpanX + pair_dx(f)];
+        weight_sum += weight;
+      }
+      if (weight_sum > 0.0f) result = static_cast<uint16_t>(lroundf(weighted_sum / weight_sum));
+    }
+    out[row * width + col] = result;
+  }
+}
+
 // VertexProjection::operator() (depth_processing.hpp:215-226), identity pose.
 __device__ __forceinline__ f3 vertex_at(const uint16_t* __restrict__ depth, int width, int x, int y,
                                         const Intr& k, const DepthParams& p) {
@@ -290,7 +371,10 @@ void Pyramid::launch(cudaStream_t s) const {
         // a window too large for the staging (48 KB) reads its pixels directly
         const size_t tile = 2 * sizeof(float) * (kTileX + 2 * static_cast<size_t>(options.bilateral_radius)) *
                             (kTileY + 2 * static_cast<size_t>(options.bilateral_radius));
-        if (tile <= 47u * 1024u) {
+        if (options.bilateral_radius == 2 && std::isfinite(p.spatial_scale) && std::isfinite(p.range_scale)) {
+          bilateral_pairs_kernel<<<dim3(ceil_div(b.width, kTileX), ceil_div(b.height, kPairRows)), 256, 0, s>>>(
+              raw.ptr, b.depth.ptr, static_cast<int>(b.width), static_cast<int>(b.height), p);
+        } else if (tile <= 47u * 1024u) {
           bilateral_kernel<true><<<grid, block, tile, s>>>(raw.ptr, b.depth.ptr, static_cast<int>(b.width),
                                                            static_cast<int>(b.height), p);
         } else {

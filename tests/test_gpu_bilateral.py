@@ -1,6 +1,7 @@
 """The bilateral filter's staged tile and table exponential against the oracle,
 bit for bit: radii whose staging spans one or several pixels per thread, a
-radius past the staging's 48 KB (read directly), sigmas that reach subnormal
+radius past the staging's 48 KB (read directly), the pairwise weights of radius
+2, sigmas that reach subnormal
 and vanishing weights, and images smaller than a tile."""
 
 import numpy as np
@@ -14,7 +15,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("width,height,radius,spatial,depth", [
-    (97, 61, 1, 2.0, 0.08), (65, 33, 7, 0.35, 0.01), (3, 2, 5, 4.0, 0.5), (70, 50, 28, 40.0, 4.0),
+    (97, 61, 1, 2.0, 0.08), (97, 61, 2, 2.0, 0.08), (33, 17, 2, 0.4, 0.004), (1, 5, 2, 3.0, 2.0), (65, 33, 7, 0.35, 0.01), (3, 2, 5, 4.0, 0.5), (70, 50, 28, 40.0, 4.0),
     (70, 50, 31, 9.0, 0.2),
 ])
 def test_bilateral_matches_oracle(width, height, radius, spatial, depth):
