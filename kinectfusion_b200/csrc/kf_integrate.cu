@@ -201,14 +201,28 @@ __global__ void cull_blocks_kernel(VolumeDev v, Rigid T, Intr k, const float* __
   if (keep) list[base + __popc(ballot & ((1u << lane) - 1u))] = block;
 }
 
+// Reciprocal (at most 1 ulp) and reciprocal square root (at most 2 ulp) of a
+// normal float, without the scaling steps that subnormals would need.
+__device__ __forceinline__ float approx_rcp(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float approx_rsqrt(float x) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
 // The pixel lround(project(K, p)) of a camera point, as observe() picks it
 // (tsdf_integration.hpp:196-205), decided without the projection's two IEEE
 // divisions where that cannot change the answer: 1 = in the image at
 // (rx, ry), -1 = no pixel (behind the camera or outside the image), 0 = too
 // close to a rounding boundary (k + 0.5) to tell - the caller then runs the
-// exact quotient.  The estimate uses __fdividef (at most 2 ulp): below 2048
-// in magnitude it is within 1.3e-3 pixel of the exact value, so a margin of
-// 4e-3 pixel decides exactly; beyond that the point is outside any image
+// exact quotient.  The estimate multiplies by an approximate reciprocal (with
+// the product's rounding at most 2 ulp of the quotient): below 2048 in
+// magnitude it is within 1.3e-3 pixel of the exact value, so a margin of 4e-3
+// pixel decides exactly; beyond that the point is outside any image
 // this path accepts (width and height up to 2048; wider images always take
 // the exact path).  Rounding to nearest even equals lround away from the
 // half-way points.
@@ -216,8 +230,9 @@ __device__ __forceinline__ int pixel_estimate(const Intr& k, f3 p, uint32_t widt
                                               uint32_t& ry) {
   if (!(p.z > 0.0f)) return -1;
   if (!(p.z >= 1e-6f) || width > 2048u || height > 2048u) return 0;
-  const float ax = __fdividef(k.fx * p.x, p.z) + k.cx;
-  const float ay = __fdividef(k.fy * p.y, p.z) + k.cy;
+  const float rz = approx_rcp(p.z);
+  const float ax = __fmaf_rn(k.fx * p.x, rz, k.cx);
+  const float ay = __fmaf_rn(k.fy * p.y, rz, k.cy);
   if (!(fabsf(ax) < 2048.0f && fabsf(ay) < 2048.0f)) return -1;
   const float nx = rintf(ax), ny = rintf(ay);
   if (fabsf(ax - nx) > 0.5f - 4e-3f || fabsf(ay - ny) > 0.5f - 4e-3f) return 0;
@@ -231,13 +246,13 @@ __device__ __forceinline__ int pixel_estimate(const Intr& k, f3 p, uint32_t widt
 // Where the projective sdf = d - |p| / lambda falls: -1 certainly below
 // -truncation (no update), +1 certainly at or above +truncation (the update
 // writes tsdf exactly 1), 0 undecided (the exact expression runs).  |p| and
-// the quotient are estimated with rsqrtf and __fdividef (relative error below
+// the quotient are estimated with approximate reciprocals (relative error below
 // 1e-6 together); the margin is 1e-4 m plus 1e-6 of the distance, far above
 // that error.
 __device__ __forceinline__ int sdf_region(f3 p, float d, float lambda, float truncation) {
   const float s2 = dot(p, p);
   if (!(s2 > 1e-30f) || !(lambda >= 1.0f)) return 0;
-  const float dist = __fdividef(s2 * rsqrtf(s2), lambda);
+  const float dist = (s2 * approx_rsqrt(s2)) * approx_rcp(lambda);
   const float est = d - dist;
   const float margin = 1e-4f + 1e-6f * dist;
   if (est < -truncation - margin) return -1;
@@ -1000,6 +1015,10 @@ void launch_pixel_table(Pipeline& p, const uint16_t* depth, const uint32_t* colo
   prepare_blocks(p, width, height, s);
   const kf_integration_options& o = p.config.integration;
   const bool tiles = o.mode != KF_INTEGRATION_BAND;  // the full sweep's block culling
+  // the integration's lists start empty: cleared here, off the pose's path
+  check(cudaMemsetAsync(p.block_count.ptr, 0, sizeof(unsigned), s), "block count clear");
+  check(cudaMemsetAsync(p.brick_dirty.ptr, 0, p.brick_dirty.bytes(), s), "dirty bits clear");
+  if (!tiles) check(cudaMemsetAsync(p.band_bits.ptr, 0, p.band_bits.bytes(), s), "band bits clear");
   pixel_table_kernel<<<dim3(ceil_div(width, kTableX), ceil_div(height, kTile)), dim3(kTableX, kTile), 0, s>>>(
       depth, color, normals, width, height, k, o.depth_scale, o.min_depth, o.max_depth, o.observation_weight,
       p.config.tsdf_rule == KF_RULE_ANGLE_WEIGHTED, table, tiles ? p.depth_tiles.ptr : nullptr, p.tile_w[0]);
@@ -1014,11 +1033,8 @@ void launch_integrate(Pipeline& p, const float4* table, uint32_t width, uint32_t
   prepare_blocks(p, width, height, s);
   const kf_integration_options& o = p.config.integration;
   const uint32_t blocks = p.view.bx * p.view.by * p.view.bz;
-  check(cudaMemsetAsync(p.block_count.ptr, 0, sizeof(unsigned), s), "block count clear");
-  check(cudaMemsetAsync(p.brick_dirty.ptr, 0, p.brick_dirty.bytes(), s), "dirty bits clear");
   if (o.mode == KF_INTEGRATION_BAND) {
     // blocks the pixels' truncation bands cross
-    check(cudaMemsetAsync(p.band_bits.ptr, 0, p.band_bits.bytes(), s), "band bits clear");
     band_mark_kernel<<<dim3(ceil_div(width, 16), ceil_div(height, 16)), dim3(16, 16), 0, s>>>(
         table, width, height, k, T, p.view.truncation, o.truncation_distance_scale, o.distance_scaled_truncation,
         p.view, state, p.band_bits.ptr);
