@@ -46,7 +46,9 @@ constexpr int kCoopLanes = 8;
 // With a ray per lane, 4 share the other lanes' gathers (1, 2, 4, 8:
 // 1001x747 render 0.491, 0.479, 0.451, 0.455 ms); with few rays per warp a
 // ray that waits for another's run only loses time (160x120 0.107 ms at 1,
-// 0.115 ms at 4).
+// 0.115 ms at 4).  A sparse march gathers most of its samples, so there the
+// runs are short and one is best (6 frames into a 2048^3 domain 8.31 ms at 1,
+// 8.58 ms at 4).
 constexpr int kRunFull = 4, kRunFew = 1;
 
 struct RaycastParams {
@@ -437,9 +439,10 @@ __device__ __forceinline__ void box_range(const VolumeDev& v, f3 o, f3 d, float&
 
 // 64 registers (16 CTAs per SM): the rounds are chains of dependent
 // instructions and lookups, so more warps hide more (1001x747 render 0.528 ms
-// at 96 registers, 0.451 at 80, 0.428 at 64 with a few spilled bytes).
+// at 96 registers, 0.451 at 80, 0.428 at 64 with a few spilled bytes); a sparse
+// march, whose gathers hold more, takes 80 (8.43 ms against 8.58 ms above).
 template <int Kind, bool Sparse>
-__global__ void __launch_bounds__(64, 16)
+__global__ void __launch_bounds__(64, Sparse ? 12 : 16)
     raycast_kernel(const __grid_constant__ VolumeDev v, SkipDev skip, RaycastParams rp, Intr k, uint32_t width, uint32_t height, Rigid pose, const IcpState* __restrict__ state, float* __restrict__ points) {
   if (state != nullptr) {
     if (state->failed) return;
@@ -953,7 +956,7 @@ void launch_typed(const Pipeline& p, const kf_raycast_camera& cam, float* points
   const uint64_t rays = static_cast<uint64_t>(cam.width) * cam.height;
   const uint32_t lanes = p.raycast_lanes[rays <= 20000u ? 0 : (rays <= 80000u ? 1 : 2)];
   rp.rays_per_warp = p.config.raycast_backend == KF_RAYCAST_BAND_MARCH ? 32u : 32u / lanes;
-  rp.run = rp.rays_per_warp == 32u ? kRunFull : kRunFew;
+  rp.run = rp.rays_per_warp == 32u && p.view.table == nullptr ? kRunFull : kRunFew;
   dim3 block(p.raycast_block_x, p.raycast_block_y);
   dim3 grid(ceil_div(cam.width, block.x), ceil_div(cam.height, block.y));
   if (rp.rays_per_warp < 32u) {
