@@ -645,7 +645,7 @@ __global__ void __launch_bounds__(64, Sparse ? 12 : 16)
 // write_surface_sample (raycasting.hpp:215-245) for every pixel whose march
 // found a zero crossing (its point is finite): the normal, then the colour
 // or the shading; without a normal the pixel has no surface.
-template <int Kind, bool Color>
+template <int Kind, bool Color, bool Sparse>
 __global__ void __launch_bounds__(128, 6)
     surface_kernel(VolumeDev v, RaycastParams rp, uint32_t width, uint32_t height, Rigid pose,
                    const IcpState* __restrict__ state, float* __restrict__ points, float* __restrict__ normals,
@@ -667,7 +667,8 @@ __global__ void __launch_bounds__(128, 6)
   uint32_t out_color = 0;
   if (finite3(surface)) {
     f3 n;
-    const bool has_normal = rp.cell_normals ? s.cell_normal(surface, n) : s.central_normal(surface, rp.policy, n);
+    const bool has_normal = rp.cell_normals ? s.template cell_normal<Sparse>(surface, n)
+                                            : s.template central_normal_of<Sparse>(surface, rp.policy, n);
     if (has_normal) {
       out_point = surface;
       out_normal = n;
@@ -995,8 +996,13 @@ void launch_typed(const Pipeline& p, const kf_raycast_camera& cam, float* points
   }
   const dim3 sblock(32, 4);
   const dim3 sgrid(ceil_div(cam.width, 32), ceil_div(cam.height, 4));
-  surface_kernel<Kind, Color><<<sgrid, sblock, 0, s>>>(p.view, rp, cam.width, cam.height, pose, state, points,
-                                                       normals, colors);
+  if (p.view.table != nullptr) {
+    surface_kernel<Kind, Color, true><<<sgrid, sblock, 0, s>>>(p.view, rp, cam.width, cam.height, pose, state, points,
+                                                               normals, colors);
+  } else {
+    surface_kernel<Kind, Color, false><<<sgrid, sblock, 0, s>>>(p.view, rp, cam.width, cam.height, pose, state,
+                                                                points, normals, colors);
+  }
   check(cudaGetLastError(), "surface_kernel launch");
 }
 

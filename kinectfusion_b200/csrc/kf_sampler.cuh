@@ -136,7 +136,7 @@ struct Sampler {
   }
 
   // tsdf() at the six points of central_normal in one pass, for the common
-  // case: dense storage, each point's stencil base one voxel from the base
+  // case: each point's stencil base one voxel from the base
   // c of the +y point's x and the +x point's y and z, along the point's own
   // axis (its other two coordinates are the centre's, so they share c's),
   // and every voxel of the plus-shaped neighbourhood (c + {-1..2} along one
@@ -145,8 +145,10 @@ struct Sampler {
   // sampler's order with its own weights, so `val` holds the values tsdf()
   // returns and `ok` is true when all six exist.  Returns false (nothing
   // decided) when the case does not apply.
+  // `Sparse` is the volume's storage, a constant of the kernel: carried at run
+  // time the two forms' registers spill (dense 640x480 normals 42 -> 53 us).
+  template <bool Sparse>
   __device__ __forceinline__ bool central_six(f3 p, int policy, float (&val)[6], bool& ok) const {
-    if (v.table != nullptr) return false;
     f3 pt[6];
     central_points(p, v.voxel_size, pt);
     f3 g[6];
@@ -180,20 +182,54 @@ struct Sampler {
         cy + 2 >= static_cast<int>(v.ry) || cz + 2 >= static_cast<int>(v.rz)) {
       return false;
     }
-    // storage_index is separable in dense storage: x, y and z terms
-    size_t tx[4], ty[4], tz[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const uint32_t x = static_cast<uint32_t>(cx - 1 + i), y = static_cast<uint32_t>(cy - 1 + i),
-                     z = static_cast<uint32_t>(cz - 1 + i);
-      tx[i] = static_cast<size_t>(x >> 3) * 512u + (x & 7u);
-      ty[i] = static_cast<size_t>(y >> 3) * v.bx * 512u + (y & 7u) * 8u;
-      tz[i] = static_cast<size_t>(z >> 3) * v.by * v.bx * 512u + (z & 7u) * 64u;
-    }
+    // storage_index is separable: the block's slot (dense storage: the block's
+    // own index), then x, y and z terms inside the block.  The neighbourhood
+    // spans at most two blocks along an axis, eight slots in all; far[a] bit i
+    // says that coordinate i of axis a lies in the second one.
     const Raw* __restrict__ vox = reinterpret_cast<const Raw*>(v.voxels);
-    // a corner's value, NaN where the sampler skips it (unobserved or not finite)
+    const uint32_t x0 = static_cast<uint32_t>(cx - 1), y0 = static_cast<uint32_t>(cy - 1),
+                   z0 = static_cast<uint32_t>(cz - 1);
+    size_t tx[4], ty[4], tz[4];
+    uint32_t far_x = 0u, far_y = 0u, far_z = 0u;
+#pragma unroll
+    for (uint32_t i = 0; i < 4; ++i) {
+      const uint32_t x = x0 + i, y = y0 + i, z = z0 + i;
+      if constexpr (!Sparse) {
+        tx[i] = static_cast<size_t>(x >> 3) * 512u + (x & 7u);
+        ty[i] = static_cast<size_t>(y >> 3) * v.bx * 512u + (y & 7u) * 8u;
+        tz[i] = static_cast<size_t>(z >> 3) * v.by * v.bx * 512u + (z & 7u) * 64u;
+      } else {
+        tx[i] = x & 7u;
+        ty[i] = (y & 7u) * 8u;
+        tz[i] = (z & 7u) * 64u;
+        far_x |= (x >> 3 != x0 >> 3 ? 1u : 0u) << i;
+        far_y |= (y >> 3 != y0 >> 3 ? 1u : 0u) << i;
+        far_z |= (z >> 3 != z0 >> 3 ? 1u : 0u) << i;
+      }
+    }
+    uint32_t slot[8];
+    if constexpr (Sparse) {
+      const uint32_t block = ((z0 >> 3) * v.by + (y0 >> 3)) * v.bx + (x0 >> 3);
+      const uint32_t sx = far_x != 0u ? 1u : 0u, sy = far_y != 0u ? v.bx : 0u, sz = far_z != 0u ? v.bx * v.by : 0u;
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        slot[c] = __ldg(v.slots + (block + (c & 1 ? sx : 0u) + (c & 2 ? sy : 0u) + (c & 4 ? sz : 0u)));
+      }
+    }
+    // a corner's value, NaN where the sampler skips it (not allocated,
+    // unobserved or not finite)
     auto value = [&](int dx, int dy, int dz) {
-      const Raw r = __ldg(vox + (tx[dx + 1] + ty[dy + 1] + tz[dz + 1]));
+      size_t at = tx[dx + 1] + ty[dy + 1] + tz[dz + 1];
+      if constexpr (Sparse) {
+        const bool fx = ((far_x >> (dx + 1)) & 1u) != 0u, fy = ((far_y >> (dy + 1)) & 1u) != 0u;
+        const bool fz = ((far_z >> (dz + 1)) & 1u) != 0u;
+        const uint32_t lo = fy ? (fx ? slot[3] : slot[2]) : (fx ? slot[1] : slot[0]);
+        const uint32_t hi = fy ? (fx ? slot[7] : slot[6]) : (fx ? slot[5] : slot[4]);
+        const uint32_t s = fz ? hi : lo;
+        if (s == kUnallocated) return __int_as_float(0x7fffffff);
+        at += static_cast<size_t>(s) * 512u;
+      }
+      const Raw r = __ldg(vox + at);
       return VT::observed(r) && VT::finite(r) ? VT::tsdf(r) : __int_as_float(0x7fffffff);
     };
     float mid[2][2][2], ax[2][2][2], ay[2][2][2], az[2][2][2];
@@ -243,10 +279,11 @@ struct Sampler {
   // trilinear::central_normal (trilinear.hpp:243-266).  The six samples
   // are independent reads of an unchanging volume, so all are taken before
   // any is tested: the result is that of the reference's early-exit order.
-  __device__ bool central_normal(f3 p, int policy, f3& out) const {
+  template <bool Sparse>
+  __device__ __forceinline__ bool central_normal_of(f3 p, int policy, f3& out) const {
     float s6[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
     bool ok = false;
-    if (!central_six(p, policy, s6, ok)) {
+    if (!central_six<Sparse>(p, policy, s6, ok)) {
       f3 pt[6];
       central_points(p, v.voxel_size, pt);
       ok = tsdf(pt[0], policy, s6[0]) & tsdf(pt[1], policy, s6[1]) & tsdf(pt[2], policy, s6[2]) &
@@ -261,7 +298,12 @@ struct Sampler {
     return true;
   }
 
+  __device__ bool central_normal(f3 p, int policy, f3& out) const {
+    return v.table != nullptr ? central_normal_of<true>(p, policy, out) : central_normal_of<false>(p, policy, out);
+  }
+
   // TrilinearSampler::cell_normal (volume_sampler.hpp:189-239)
+  template <bool Sparse>
   __device__ bool cell_normal(f3 p, f3& out) const {
     const f3 g = grid_of(p);
     if (!contains(g)) return false;
@@ -277,9 +319,9 @@ struct Sampler {
 #pragma unroll
         for (int ox = 0; ox <= 1; ++ox) {
           const Raw* cp = corner(bx + ox, by + oy, bz + oz);
-          if (cp == nullptr) return central_normal(p, KF_CORNERS_SKIP_MISSING, out);
+          if (cp == nullptr) return central_normal_of<Sparse>(p, KF_CORNERS_SKIP_MISSING, out);
           const Raw r = __ldg(cp);
-          if (!VT::observed(r) || !VT::finite(r)) return central_normal(p, KF_CORNERS_SKIP_MISSING, out);
+          if (!VT::observed(r) || !VT::finite(r)) return central_normal_of<Sparse>(p, KF_CORNERS_SKIP_MISSING, out);
           c[oz][oy][ox] = VT::tsdf(r);
         }
       }
