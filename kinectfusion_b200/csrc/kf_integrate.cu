@@ -565,45 +565,49 @@ __global__ void stencil_bits_kernel(const uint4* __restrict__ voxel_bits, uint4*
 // bricks past the brick grid count as different, so the cube stays inside
 // it.  Mixed bricks get 0.  The raycast crosses such a cube in one go, as it
 // crosses a single brick of that class.  Three separable passes, one per
-// axis: `lower` (the previous pass's radius: the run along x, then the
-// square in x and y) bounds the radius at every brick of the new axis'
-// segment; the x pass has none.
+// axis: the previous pass's radius (the run along x, then the square in x and
+// y) bounds the radius at every brick of the new axis' segment; the x pass has
+// none.  Every pass reads and writes codes (class | radius << 2; the x pass
+// reads the classes, codes of radius 0), so a brick is one byte to load:
+// 16.3 us for the three at 512^3, 20.7 us with the class and the bound apart.
 constexpr uint32_t kBrickRadiusCap = 7;
-__global__ void brick_radius_kernel(const uint8_t* __restrict__ brick_class, const uint8_t* __restrict__ lower,
-                                    uint8_t* __restrict__ out, uint32_t bx, uint32_t by, uint32_t bz, int axis,
-                                    const IcpState* __restrict__ state) {
-  // the last pass writes the brick's code (class | radius << 2)
+template <int Axis>
+__global__ void __launch_bounds__(256)
+    brick_radius_kernel(const uint8_t* __restrict__ in, uint8_t* __restrict__ out, uint32_t bx, uint32_t by,
+                        uint32_t bz, const IcpState* __restrict__ state) {
   if (state != nullptr && state->failed) return;  // no integration this frame: the classes stand
   const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= bx * by * bz) return;
-  const uint32_t c = brick_class[b];
-  if (c != 1u && c != 2u) {
-    out[b] = static_cast<uint8_t>(axis == 2 ? c : 0u);
+  const uint32_t mine = __ldg(in + b), c = mine & 3u;
+  if (c == 0u) {
+    out[b] = 0u;
     return;
   }
-  const uint32_t coord = axis == 0 ? b % bx : (axis == 1 ? (b / bx) % by : b / (bx * by));
-  const uint32_t extent = axis == 0 ? bx : (axis == 1 ? by : bz);
-  const size_t stride = axis == 0 ? 1u : (axis == 1 ? bx : static_cast<size_t>(bx) * by);
+  const uint32_t coord = Axis == 0 ? b % bx : (Axis == 1 ? (b / bx) % by : b / (bx * by));
+  const uint32_t extent = Axis == 0 ? bx : (Axis == 1 ? by : bz);
+  const uint32_t stride = Axis == 0 ? 1u : (Axis == 1 ? bx : bx * by);
   // r = the first k that fails, less one: both neighbours at distance k
   // inside the grid and of class c, and (later passes) k within the bound
   // of every brick passed so far.  Every distance's loads are independent
   // of the others' outcome, so all are issued before the scan.
-  uint32_t m = lower != nullptr ? lower[b] : kBrickRadiusCap;
+  uint32_t lo[kBrickRadiusCap], hi[kBrickRadiusCap];
+#pragma unroll
+  for (uint32_t k = 1; k <= kBrickRadiusCap; ++k) {
+    const bool inside = coord >= k && coord + k < extent;
+    lo[k - 1] = inside ? __ldg(in + (b - k * stride)) : 0u;  // past the grid: another class
+    hi[k - 1] = inside ? __ldg(in + (b + k * stride)) : 0u;
+  }
+  uint32_t m = Axis == 0 ? kBrickRadiusCap : mine >> 2;
   uint32_t r = 0;
   bool run = true;
 #pragma unroll
   for (uint32_t k = 1; k <= kBrickRadiusCap; ++k) {
-    const bool in = coord >= k && coord + k < extent;
-    const size_t lo = in ? b - k * stride : b, hi = in ? b + k * stride : b;
-    const uint32_t cl = brick_class[lo], ch = brick_class[hi];
-    const uint32_t ml = lower != nullptr ? lower[lo] : kBrickRadiusCap;
-    const uint32_t mh = lower != nullptr ? lower[hi] : kBrickRadiusCap;
-    run = run && k <= m && in && cl == c && ch == c;
-    if (run) m = min(m, min(ml, mh));
+    run = run && k <= m && (lo[k - 1] & 3u) == c && (hi[k - 1] & 3u) == c;
+    if (Axis != 0 && run) m = min(m, min(lo[k - 1] >> 2, hi[k - 1] >> 2));
     run = run && !(m < k);
     if (run) r = k;
   }
-  out[b] = static_cast<uint8_t>(axis == 2 ? (c | (r << 2)) : r);
+  out[b] = static_cast<uint8_t>(c | (r << 2));
 }
 
 // ---- band integration (BandIntegrationSweep<kDevice>, tsdf_integration.cu:
@@ -1110,12 +1114,11 @@ void launch_integrate(Pipeline& p, const float4* table, uint32_t width, uint32_t
   const uint32_t bricks = static_cast<uint32_t>(p.brick_code.count);
   uint8_t* run_x = p.radius_scratch.ptr;
   uint8_t* square_xy = p.radius_scratch.ptr + bricks;
-  brick_radius_kernel<<<ceil_div(bricks, 256u), 256, 0, s>>>(p.brick_class.ptr, nullptr, run_x, p.view.bx, p.view.by,
-                                                              p.view.bz, 0, state);
-  brick_radius_kernel<<<ceil_div(bricks, 256u), 256, 0, s>>>(p.brick_class.ptr, run_x, square_xy, p.view.bx,
-                                                              p.view.by, p.view.bz, 1, state);
-  brick_radius_kernel<<<ceil_div(bricks, 256u), 256, 0, s>>>(p.brick_class.ptr, square_xy, p.brick_code.ptr,
-                                                              p.view.bx, p.view.by, p.view.bz, 2, state);
+  const unsigned radius_ctas = ceil_div(bricks, 256u);
+  brick_radius_kernel<0><<<radius_ctas, 256, 0, s>>>(p.brick_class.ptr, run_x, p.view.bx, p.view.by, p.view.bz, state);
+  brick_radius_kernel<1><<<radius_ctas, 256, 0, s>>>(run_x, square_xy, p.view.bx, p.view.by, p.view.bz, state);
+  brick_radius_kernel<2><<<radius_ctas, 256, 0, s>>>(square_xy, p.brick_code.ptr, p.view.bx, p.view.by, p.view.bz,
+                                                     state);
   check(cudaGetLastError(), "brick_radius_kernel launch");
 }
 
