@@ -122,9 +122,11 @@ __global__ void __launch_bounds__(kTileX* kTileY)
   if (center == center) {
     float weighted_sum = 0.0f;
     float weight_sum = 0.0f;
-    // pixels outside the image are NaN: skipped, as the reference's clipped window
-    for (int dy = -p.radius; dy <= p.radius; ++dy) {
-      for (int dx = -p.radius; dx <= p.radius; ++dx) {
+    // the reference's window, clipped to the image
+    const int x0 = max(-p.radius, -col), x1 = min(p.radius, width - 1 - col);
+    const int y0 = max(-p.radius, -row), y1 = min(p.radius, height - 1 - row);
+    for (int dy = y0; dy <= y1; ++dy) {
+      for (int dx = x0; dx <= x1; ++dx) {
         float sample, raw;
         staged(dx, dy, sample, raw);
         if (sample != sample) continue;
@@ -358,7 +360,10 @@ uint32_t Pyramid::prepare(uint32_t w, uint32_t h, kf_intrinsics k) {
 }
 
 void Pyramid::launch(cudaStream_t s) const {
-  const DepthParams p = depth_params(options);
+  DepthParams p = depth_params(options);
+  // no window reaches past the image: any non-negative radius is accepted, and
+  // the filter's sizes and indices stay those of the image
+  p.radius = std::min(p.radius, static_cast<int>(std::max(width, height)) - 1);
   for (uint32_t level = 0; level < level_count; ++level) {
     const PyramidLevelBuffers& b = levels[level];
     const dim3 block(kTileX, kTileY);
@@ -369,8 +374,8 @@ void Pyramid::launch(cudaStream_t s) const {
               "pyramid level-0 copy");
       } else {
         // a window too large for the staging (48 KB) reads its pixels directly
-        const size_t tile = 2 * sizeof(float) * (kTileX + 2 * static_cast<size_t>(options.bilateral_radius)) *
-                            (kTileY + 2 * static_cast<size_t>(options.bilateral_radius));
+        const size_t tile = 2 * sizeof(float) * (kTileX + 2 * static_cast<size_t>(p.radius)) *
+                            (kTileY + 2 * static_cast<size_t>(p.radius));
         if (options.bilateral_radius == 2 && std::isfinite(p.spatial_scale) && std::isfinite(p.range_scale)) {
           bilateral_pairs_kernel<<<dim3(ceil_div(b.width, kTileX), ceil_div(b.height, kPairRows)), 256, 0, s>>>(
               raw.ptr, b.depth.ptr, static_cast<int>(b.width), static_cast<int>(b.height), p);
