@@ -376,7 +376,10 @@ void Pyramid::launch(cudaStream_t s) const {
         // a window too large for the staging (48 KB) reads its pixels directly
         const size_t tile = 2 * sizeof(float) * (kTileX + 2 * static_cast<size_t>(p.radius)) *
                             (kTileY + 2 * static_cast<size_t>(p.radius));
-        if (options.bilateral_radius == 2 && std::isfinite(p.spatial_scale) && std::isfinite(p.range_scale)) {
+        // pairs: scales and metres all finite, so that a pair's weight is the
+        // same number from both ends and the centre's is exactly 1
+        if (options.bilateral_radius == 2 && std::isfinite(p.spatial_scale) && std::isfinite(p.range_scale) &&
+            std::isfinite(65535.0f / p.depth_scale)) {
           bilateral_pairs_kernel<<<dim3(ceil_div(b.width, kTileX), ceil_div(b.height, kPairRows)), 256, 0, s>>>(
               raw.ptr, b.depth.ptr, static_cast<int>(b.width), static_cast<int>(b.height), p);
         } else if (tile <= 47u * 1024u) {
