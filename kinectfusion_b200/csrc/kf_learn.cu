@@ -23,17 +23,11 @@
 #include <vector>
 
 #include "kf_internal.h"
+#include "kf_learn_shape.h"
 
 namespace kf {
 namespace {
 
-struct Conv {
-  int cin, cout, hin, win, hout, wout, k, kpad;
-};
-constexpr Conv kConv[4] = {{2, 32, 60, 80, 30, 40, 18, 24},
-                           {32, 32, 30, 40, 15, 20, 288, 288},
-                           {32, 64, 15, 20, 8, 10, 288, 288},
-                           {64, 64, 8, 10, 4, 5, 576, 576}};
 constexpr int kFlat = 64 * 4 * 5;  // 1280
 constexpr int kHidden = 256;
 constexpr int kOut = 6;
@@ -74,11 +68,13 @@ __global__ void __launch_bounds__(256)
     im2col_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ col, int batch) {
   constexpr Conv c = kConv[L];
   static_assert(c.kpad % 8 == 0, "whole 16-byte stores");
-  const int i = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x);
-  if (i >= batch * (c.hout * c.wout * (c.kpad / 8))) return;
-  const int k0 = i % (c.kpad / 8) * 8, row = i / (c.kpad / 8);
-  const int ox = row % c.wout, oy = (row / c.wout) % c.hout, b = row / (c.wout * c.hout);
-  const unsigned short* in = reinterpret_cast<const unsigned short*>(x) + b * (c.hin * c.win * c.cin);
+  // 32 bits count the threads: at most 10,800 a sample
+  const unsigned i = blockIdx.x * 256u + threadIdx.x;
+  if (i >= static_cast<size_t>(batch) * (column_values(c) / 8u)) return;
+  const int k0 = i % (c.kpad / 8) * 8;
+  const unsigned row = i / (c.kpad / 8);
+  const int ox = row % c.wout, oy = (row / c.wout) % c.hout;
+  const unsigned short* in = reinterpret_cast<const unsigned short*>(x) + input_at(c, row / (c.wout * c.hout));
   unsigned short v[8];
 #pragma unroll
   for (int u = 0; u < 8; ++u) {
@@ -100,10 +96,14 @@ template <int L>
 __global__ void __launch_bounds__(256)
     col2im_kernel(const float* __restrict__ dcol, float* __restrict__ dx, int batch) {
   constexpr Conv c = kConv[L];
-  const int i = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x);
-  if (i >= batch * (c.hin * c.win * c.cin)) return;
-  const int ch = i % c.cin, p = i / c.cin;
-  const int x = p % c.win, y = (p / c.win) % c.hin, b = p / (c.win * c.hin);
+  // 32 bits count the threads: at most 38,400 a sample of a batch that
+  // colsum_chunks allows
+  const unsigned i = blockIdx.x * 256u + threadIdx.x;
+  if (i >= static_cast<size_t>(batch) * input_values(c)) return;
+  const int ch = i % c.cin;
+  const unsigned p = i / c.cin;
+  const int x = p % c.win, y = (p / c.win) % c.hin;
+  const float* in_sample = dcol + column_at(c, p / (c.win * c.hin));
   // at most two window rows and columns reach the element: their loads are
   // issued together, then added in the windows' order
   float v[9];
@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(256)
   for (int k = 0; k < 9; ++k) {
     const int ty = y + 1 - k / 3, tx = x + 1 - k % 3, oy = ty >> 1, ox = tx >> 1;
     const bool in = ty >= 0 && tx >= 0 && ((ty | tx) & 1) == 0 && oy < c.hout && ox < c.wout;
-    v[k] = in ? __ldg(dcol + ((b * c.hout + oy) * c.wout + ox) * c.kpad + ch * 9 + k) : 0.0f;
+    v[k] = in ? __ldg(in_sample + (oy * c.wout + ox) * c.kpad + ch * 9 + k) : 0.0f;
   }
   float s = 0.0f;
 #pragma unroll
@@ -168,7 +168,6 @@ __global__ void transpose_weights_kernel(WeightTransposes w) {
 // column sums of dz over chunks of 256 rows, each in a fixed order, into
 // partial[chunk][c].  (Masking, rounding, transposing and summing in four
 // kernels took 44 us for conv1 at batch 64, 21.7 us.)
-constexpr int kColsumRows = 256;
 __global__ void __launch_bounds__(256)
     dz_kernel(const float* __restrict__ dy, const float* __restrict__ a, int rows, int cols,
               __nv_bfloat16* __restrict__ rows_out, __nv_bfloat16* __restrict__ cols_out, int out_ld,
@@ -443,6 +442,11 @@ struct Learner {
 
   // gradients of the batch-mean squared twist error into grads (after forward)
   void backward(const float* target, int batch, cudaStream_t s) {
+    // the widest layer's bias sums would not fit a grid: refused before any
+    // kernel of the pass runs
+    if (colsum_chunks(kConv[0], static_cast<unsigned>(batch)) > kMaxColsumChunks) {
+      throw CudaError("learner backward: the batch needs more than 65535 chunks of bias sums");
+    }
     loss_kernel<<<1, 256, 0, s>>>(out.ptr, target, batch, dout8.ptr, loss.ptr);
     // fc2: dW = d_out^T x5 (the first 6 rows of an 8-row product), db, dx5 = d_out W
     layer_grads(dout8.ptr, nullptr, batch, kOutPad, xbf[5].ptr, kHidden, true, dcol.ptr, grads.ptr + lay.b[5], kOut,
