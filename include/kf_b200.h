@@ -430,8 +430,10 @@ kf_status kf_tracker_destroy(kf_tracker* tracker);
  * This arms the tracker so that the exchange of its next level never
  * completes (it waits for tags nobody writes): the waits run out, the frame
  * is marked failed (no integration), and the call that reads the result
- * returns KF_ERR_DEVICE_TIMEOUT and clears the exchange, after which the
- * tracker runs normally.  Call it with no work of the tracker in flight. */
+ * returns KF_ERR_DEVICE_TIMEOUT and restarts the exchange, after which the
+ * tracker runs normally.  Frames submitted before that call fail the same
+ * way: none of them is tracked or fused.  Call it with no work of the tracker
+ * in flight. */
 kf_status kf_tracker_stall_next_level(kf_tracker* tracker);
 /* Renders the model at `camera` and tracks `live` against it for `iterations`
  * Gauss-Newton steps starting from camera->camera_to_world

@@ -994,14 +994,25 @@ __global__ void __launch_bounds__(kIcpBlock, 1)
   __shared__ CombineShared s_combine;
   __shared__ IcpState s_st;
   __shared__ float s_tested[kIcpSums];
+  __shared__ unsigned s_broken;
   constexpr unsigned kWords = offsetof(IcpState, barrier) / sizeof(unsigned);
   static_assert(offsetof(IcpState, barrier) % sizeof(unsigned) == 0, "state words");
   {
     const unsigned* src = reinterpret_cast<const unsigned*>(st);
     unsigned* dst = reinterpret_cast<unsigned*>(&s_st);
     for (unsigned w = threadIdx.x; w < kWords; w += kIcpBlock) dst[w] = src[w];
+    if (threadIdx.x == 0) s_broken = load_acquire(&st->barrier.broken);
   }
   __syncthreads();
+  if (s_broken != 0u) {
+    // An exchange of this tracker gave up and the host has not restarted it
+    // yet (icp_exchange_restart_kernel): the tags stand where that level
+    // began, so its packets would pass for this level's.  The frame fails; a
+    // CTA that started before the mark finds no packet of this one and gives
+    // up too.
+    if (threadIdx.x == 0) st->failed = 1;
+    return;
+  }
   if (threadIdx.x == 0 && begin) level_begin(&s_st, p.damping_lambda);
   if (threadIdx.x == 0) s_tested[0] = kNaN;  // no step has tested its system yet
   // the first step's tag (set by the previous launch's CTA 0 after its last
@@ -1051,7 +1062,23 @@ __global__ void __launch_bounds__(kIcpBlock, 1)
   __syncthreads();
   const unsigned* src = reinterpret_cast<const unsigned*>(&s_st);
   unsigned* dst = reinterpret_cast<unsigned*>(st);
-  for (unsigned w = threadIdx.x; w < kWords; w += kIcpBlock) dst[w] = src[w];
+  // a CTA whose wait gave up in the last step has marked the frame failed: that
+  // mark stands (a level starts with it clear, or ends with it set)
+  constexpr unsigned kFailedWord = offsetof(IcpState, failed) / sizeof(unsigned);
+  const bool failed = s_st.failed != 0;
+  for (unsigned w = threadIdx.x; w < kWords; w += kIcpBlock) {
+    if (w != kFailedWord || failed) dst[w] = src[w];
+  }
+}
+
+// Restarts the exchange of a tracker one of whose waits gave up, on the
+// device and from the device's own step count: frames that ran since the host
+// took its copy may have moved it.
+__global__ void icp_exchange_restart_kernel(IcpBarrier* b) {
+  if (threadIdx.x != 0 || b->broken == 0u) return;
+  b->base += kIcpStepGap;
+  b->broken = 0u;
+  b->stall = 0u;
 }
 
 __global__ void icp_level_begin_kernel(IcpState* st, float damping_lambda) {
@@ -1211,11 +1238,9 @@ void launch_icp_level(const IcpLevelArgs& args, IcpState* state, float* partials
 
 void check_icp_barrier(const IcpState& host, IcpState* device, cudaStream_t s) {
   if (host.barrier.broken == 0u) return;
-  const IcpBarrier fresh{host.barrier.base + kIcpStepGap, 0u, 0u};
-  check(cudaMemcpyAsync(reinterpret_cast<char*>(device) + offsetof(IcpState, barrier), &fresh, sizeof(fresh),
-                        cudaMemcpyHostToDevice, s),
-        "ICP barrier reset");
-  check(cudaStreamSynchronize(s), "ICP barrier reset");
+  icp_exchange_restart_kernel<<<1, 32, 0, s>>>(&device->barrier);
+  check(cudaGetLastError(), "ICP exchange restart");
+  check(cudaStreamSynchronize(s), "ICP exchange restart");
   throw DeviceTimeout(
       "ICP level kernel: a grid-barrier wait gave up before every CTA arrived; the frame is marked failed");
 }

@@ -170,8 +170,10 @@ constexpr int kIcpRunning = -1;
 
 // The step exchange of the whole-level ICP kernel: the steps exchanged since
 // the tracker's creation, whose low 32 bits tag the packets of the next one;
-// a sticky give-up flag set by a wait that ran out of time; and the test
-// hook's flag, which makes the next level wait for tags nobody writes.
+// a give-up flag set by a wait that ran out of time, under which every later
+// level fails its frame until the host has read a result that shows it
+// (check_icp_barrier); and the test hook's flag, which makes the next level
+// wait for tags nobody writes.
 struct IcpBarrier {
   unsigned long long base;
   unsigned broken;
@@ -279,8 +281,9 @@ void launch_icp_level(const IcpLevelArgs& args, IcpState* state, float* partials
 // combine and step); for frame graphs that run beside others (batches).
 void launch_icp_level_steps(const IcpLevelArgs& args, IcpState* state, float* partials, const IcpParams& params,
                             uint32_t iterations, int level, cudaStream_t stream);
-// Throws DeviceTimeout when the downloaded state `host` shows a grid barrier
-// that gave up; the device barrier is cleared first (ordered on `stream`).
+// Throws DeviceTimeout when the downloaded state `host` shows an exchange that
+// gave up, its own frame's or an earlier one's; the device's exchange is
+// restarted first if it still stands broken (ordered on `stream`).
 void check_icp_barrier(const IcpState& host, IcpState* device, cudaStream_t stream);
 // kf_icp_level's start: the pose, the level start, and the given model
 // transform in place of the pose's inverse.
