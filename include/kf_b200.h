@@ -519,7 +519,8 @@ kf_status kf_frame_result_fetch(kf_pipeline* pipeline, kf_frame_result* result);
  * copy of the frame's result into a queue of eight; host inputs are staged
  * while earlier frames still run.  kf_frame_result_next waits for the oldest
  * queued frame only and returns its result; submitting a ninth frame before
- * reading one is KF_ERR_INVALID_ARGUMENT. */
+ * reading one is KF_ERR_INVALID_ARGUMENT.  A result that is an error
+ * (KF_ERR_DEVICE_TIMEOUT) has left the queue too. */
 kf_status kf_frame_submit(kf_pipeline* pipeline, kf_pyramid* pyramid, kf_tracker* tracker,
                           const uint16_t* depth, const uint32_t* color, uint32_t width,
                           uint32_t height, kf_intrinsics intrinsics, int32_t memory,

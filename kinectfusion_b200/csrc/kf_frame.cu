@@ -279,8 +279,9 @@ void enqueue(kf_pipeline* pipeline, kf_pyramid* pyramid, kf_tracker* tracker, co
   p.last_frame_kernels = fg.kernels;
 }
 
-// `device` is the tracker state the frame ran on: a grid barrier that gave
-// up during the frame is cleared there and reported as an error.
+// `device` is the tracker state the frame ran on: an exchange that gave up
+// during the frame, or before it and not yet reported, is restarted there and
+// reported as an error.
 void fill_result(const IcpState& st, int first, kf_frame_result* r, IcpState* device, cudaStream_t s) {
   if (device != nullptr) check_icp_barrier(st, device, s);
   for (int i = 0; i < 3; ++i) {
@@ -499,9 +500,11 @@ kf_status kf_frame_result_next(kf_pipeline* pipeline, kf_frame_result* result) {
     require(p.results_popped < p.results_pushed, "kf_frame_result_next: no submitted frame is waiting");
     const int slot = static_cast<int>(p.results_popped % Pipeline::kResultSlots);
     check(cudaEventSynchronize(p.result_ready[slot]), "frame");
-    fill_result(p.result_ring.ptr[slot], p.result_first[slot], result,
-                p.graph_tracker ? p.graph_tracker->impl.state.ptr : nullptr, p.stream);
+    // out of the queue first: a result that is an error has been read too
+    const IcpState state = p.result_ring.ptr[slot];
     ++p.results_popped;
+    fill_result(state, p.result_first[slot], result, p.graph_tracker ? p.graph_tracker->impl.state.ptr : nullptr,
+                p.stream);
   });
 }
 

@@ -115,3 +115,20 @@ def test_a_late_read_moves_nothing_back(seq, clean):
     loop.enqueue(3)
     assert np.array_equal(pose(*loop.fetch()), poses[3])
     assert np.array_equal(loop.pipeline.download_raw().view(np.uint32), volumes[3])
+
+
+def test_an_error_leaves_the_result_queue(seq, clean):
+    poses, volumes = clean
+    loop = start(seq, clean)
+    fused = loop.updates()
+    for f in (2, 3, 2, 3, 2, 3, 2, 3):
+        loop.submit(f)  # eight results wait: the queue is full
+    for _ in range(8):
+        assert loop.next()[0] == abi.KF_ERR_DEVICE_TIMEOUT
+    assert loop.next()[0] == abi.KF_ERR_INVALID_ARGUMENT  # nothing waits any more
+    assert loop.updates() == fused
+    loop.submit(2)
+    loop.submit(3)
+    for f in (2, 3):
+        assert np.array_equal(pose(*loop.next()), poses[f])
+    assert np.array_equal(loop.pipeline.download_raw().view(np.uint32), volumes[3])
