@@ -284,7 +284,8 @@ kf_status kf_pipeline_integrate(kf_pipeline* pipeline, const kf_frame_view* fram
 /* Pipeline::raycast (pipeline.hpp:81): renders into `out` (host or device buffers). */
 kf_status kf_pipeline_raycast(kf_pipeline* pipeline, const kf_raycast_camera* camera,
                               const kf_surface_maps* out);
-/* Pipeline::observed_voxel_count (pipeline.hpp:87). */
+/* Pipeline::observed_voxel_count (pipeline.hpp:87).  Counts and meshes of one
+ * pipeline may be asked for from several threads; the calls take turns. */
 kf_status kf_pipeline_observed_voxel_count(kf_pipeline* pipeline, uint64_t* count);
 /* Pipeline::host_view (pipeline.hpp:90): dense float staging copy.  tsdf and
  * weight are voxel_count floats; color (voxel_count*4 floats) may be NULL. */
@@ -331,7 +332,8 @@ kf_status kf_pipeline_download_pool(kf_pipeline* pipeline, void* voxels, size_t 
  * ceil(blocks / 32) words. */
 kf_status kf_pipeline_download_band_bitmap(kf_pipeline* pipeline, uint32_t* words, size_t count);
 
-/* Pipeline::extract_mesh (pipeline.hpp:95) on the device; free with kf_mesh_free. */
+/* Pipeline::extract_mesh (pipeline.hpp:95) on the device; free with
+ * kf_mesh_free.  Threads: as kf_pipeline_observed_voxel_count. */
 kf_status kf_pipeline_extract_mesh(kf_pipeline* pipeline, float min_weight, kf_mesh* out);
 void kf_mesh_free(kf_mesh* mesh);
 /* Waits for the pipeline's stream. */

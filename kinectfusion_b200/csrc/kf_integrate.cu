@@ -1174,6 +1174,7 @@ void launch_refill_volume(Pipeline& p, cudaStream_t s) {
 }
 
 uint64_t count_observed(Pipeline& p) {
+  const std::lock_guard<std::mutex> lock(p.reading);  // the count's word is the pipeline's
   Touched t;
   if (!touched_bricks(p, t)) {
     check(cudaStreamSynchronize(p.stream), "count observed");

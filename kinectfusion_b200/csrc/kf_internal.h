@@ -5,6 +5,7 @@
 #include <stdint.h>
 
 #include <map>
+#include <mutex>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -357,6 +358,9 @@ struct Pipeline {
   };
   std::map<std::pair<uint32_t, uint32_t>, Maps> maps;
   cudaStream_t stream = nullptr;
+  // Working memory of the calls that only read the volume and that several
+  // threads may make at once: each of them holds `reading` throughout.
+  std::mutex reading;
   // kf_pipeline_extract_mesh's working arrays and page-locked staging
   DeviceArray<uint8_t> mesh_cells, mesh_surface;
   PinnedArray<uint8_t> mesh_staging;

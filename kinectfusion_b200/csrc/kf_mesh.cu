@@ -588,6 +588,7 @@ void extract_typed(Pipeline& p, float min_weight, kf_mesh& out, cudaStream_t s) 
 void extract_mesh(Pipeline& p, float min_weight, kf_mesh& out) {
   std::memset(&out, 0, sizeof(out));
   if (p.view.rx < 2 || p.view.ry < 2 || p.view.rz < 2) return;
+  const std::lock_guard<std::mutex> lock(p.reading);  // the working arrays are the pipeline's
   const cudaStream_t s = p.stream;
   try {
     switch (p.config.voxel) {
