@@ -25,7 +25,8 @@
 //     average, summed in triangle order as the host builder does.
 //
 // The working arrays stay with the pipeline between calls (up to
-// kMeshKeepBytes), and the mesh comes back through page-locked staging.
+// kMeshKeepBytes in all), and the mesh comes back through page-locked staging
+// (up to kMeshStageBytes; a larger one is copied straight to its arrays).
 // 512^3 float after 8 frames: 0.86 ms a call against 6.7 ms with a pass
 // over every cell, twenty allocations and the fill on the host.
 #include <algorithm>
@@ -425,23 +426,21 @@ struct Scratch {
   static size_t bytes(size_t n) { return (n * sizeof(uint32_t) + 255) / 256 * 256; }  // n words
 };
 
-// A larger working buffer is given back at the end of the call.
+// What a pipeline keeps of the working memory after a call: this much device
+// memory in all and this much page-locked memory.  The rest is given back.
 constexpr size_t kMeshKeepBytes = size_t{256} << 20;
+constexpr size_t kMeshStageBytes = size_t{64} << 20;
 
 void reserve(DeviceArray<uint8_t>& buffer, size_t bytes) {
   if (buffer.count < bytes) buffer.resize(bytes);
 }
 
-// Gives the buffers back when they are larger than a pipeline should keep.
+// Gives back what a pipeline should not keep.
 struct TrimMeshBuffers {
   Pipeline& p;
   ~TrimMeshBuffers() {
-    for (DeviceArray<uint8_t>* b : {&p.mesh_cells, &p.mesh_surface}) {
-      if (b->count > kMeshKeepBytes) {
-        b->release();
-      }
-    }
-    if (p.mesh_staging.count > kMeshKeepBytes) p.mesh_staging.release();
+    if (p.mesh_cells.count > kMeshKeepBytes) p.mesh_cells.release();
+    if (p.mesh_cells.count + p.mesh_surface.count > kMeshKeepBytes) p.mesh_surface.release();
   }
 };
 
@@ -550,9 +549,10 @@ void extract_typed(Pipeline& p, float min_weight, kf_mesh& out, cudaStream_t s) 
   mc_fill_normals_kernel<<<ceil_div(vertices, 128), 128, 0, s>>>(positions, tris, incident, incident_list, vertices,
                                                                  normals);
   check(cudaGetLastError(), "mc_fill_normals_kernel launch");
-  // to the host through page-locked staging
+  // to the host, through page-locked staging unless the mesh is larger than it
   const size_t vertex_bytes = three * sizeof(float), triangle_bytes = static_cast<size_t>(corners) * sizeof(uint32_t);
-  p.mesh_staging.resize(3 * vertex_bytes + triangle_bytes);
+  const bool stage = 3 * vertex_bytes + triangle_bytes <= kMeshStageBytes;
+  if (stage) p.mesh_staging.resize(3 * vertex_bytes + triangle_bytes);
   uint8_t* staged = p.mesh_staging.ptr;
   out.vertex_count = vertices;
   out.triangle_count = triangles;
@@ -565,17 +565,28 @@ void extract_typed(Pipeline& p, float min_weight, kf_mesh& out, cudaStream_t s) 
                          {normals, reinterpret_cast<void**>(&out.normals), vertex_bytes},
                          {colors, reinterpret_cast<void**>(&out.colors), vertex_bytes},
                          {tris, reinterpret_cast<void**>(&out.triangles), triangle_bytes}};
-  for (const Part& part : parts) {
-    check(cudaMemcpyAsync(staged, part.device, part.bytes, cudaMemcpyDeviceToHost, s), "mesh copy");
-    staged += part.bytes;
+  if (stage) {
+    for (const Part& part : parts) {
+      check(cudaMemcpyAsync(staged, part.device, part.bytes, cudaMemcpyDeviceToHost, s), "mesh copy");
+      staged += part.bytes;
+    }
   }
   bool allocated = true;
   for (const Part& part : parts) {
     *part.host = std::malloc(part.bytes);
     allocated = allocated && *part.host != nullptr;
   }
+  if (!allocated) {
+    cudaStreamSynchronize(s);
+    throw CudaError("host allocation failed");
+  }
+  if (!stage) {
+    for (const Part& part : parts) {
+      check(cudaMemcpyAsync(*part.host, part.device, part.bytes, cudaMemcpyDeviceToHost, s), "mesh copy");
+    }
+  }
   check(cudaStreamSynchronize(s), "mesh copy");
-  if (!allocated) throw CudaError("host allocation failed");
+  if (!stage) return;
   staged = p.mesh_staging.ptr;
   for (const Part& part : parts) {
     std::memcpy(*part.host, staged, part.bytes);
