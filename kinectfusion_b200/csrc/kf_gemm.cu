@@ -20,6 +20,7 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
+#include <atomic>
 #include <mutex>
 
 #include "kf_internal.h"
@@ -30,6 +31,7 @@ namespace {
 constexpr int kGemmThreads = 128;
 constexpr int kGemmBM = 128;
 constexpr int kGemmBK = 64;
+constexpr int kGemmDevices = 64;  // devices whose kernel attributes are remembered
 constexpr unsigned long long kWaitCycles = 2000000000ull;  // ~1 s at 2 GHz
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
@@ -317,12 +319,15 @@ template <int BN>
 void launch_tiles(const __nv_bfloat16* a, const __nv_bfloat16* b, float* c, int M, int N, int K, int lda, int ldb,
                   int ldc, const float* bias, int relu, int slabs, unsigned splits, int* error, __nv_bfloat16* out_bf16,
                   cudaStream_t s) {
-  static bool configured = false;  // per process: every device gets the same attribute
-  if (!configured) {
+  // the shared-memory limit is an attribute of the kernel on one device
+  static std::atomic<bool> configured[kGemmDevices];
+  int device = 0;
+  check(cudaGetDevice(&device), "gemm device");
+  if (device >= kGemmDevices || !configured[device].load(std::memory_order_acquire)) {
     check(cudaFuncSetAttribute(gemm_bf16_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                static_cast<int>(gemm_smem_bytes<BN>())),
           "gemm attribute");
-    configured = true;
+    if (device < kGemmDevices) configured[device].store(true, std::memory_order_release);
   }
   const CUtensorMap ma = tensor_map(a, M, K, lda, kGemmBM);
   const CUtensorMap mb = tensor_map(b, N, K, ldb, BN);
