@@ -1,6 +1,7 @@
 // kf_api.cu - C ABI entry points (include/kf_b200.h) for pipelines, trackers
 // and the whole-frame CUDA graph.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <string>
@@ -108,6 +109,11 @@ void check(cudaError_t status, const char* what) {
 
 void require(bool condition, const char* what) {
   if (!condition) throw InvalidArgument(what);
+}
+
+uint64_t next_generation() {
+  static std::atomic<uint64_t> last{0};
+  return ++last;
 }
 
 Pipeline::Maps& Pipeline::maps_for(uint32_t w, uint32_t h) {
@@ -365,7 +371,10 @@ kf_status kf_pipeline_integrate(kf_pipeline* pipeline, const kf_frame_view* fram
     const uint16_t* depth = stage(f.depth, n, f.memory, p.own_depth, p.stream);
     const uint32_t* color = stage(f.color, n, f.memory, p.own_color, p.stream);
     const float* normals = stage(f.normals, n * 3, f.memory, p.own_normals, p.stream);
-    if (p.pixel_table.count != n) p.pixel_table.resize(n);
+    if (p.pixel_table.count != n) {
+      p.generation = next_generation();
+      p.pixel_table.resize(n);
+    }
     const Intr k = intr_from(f.intrinsics);
     launch_pixel_table(p, depth, color, normals, f.width, f.height, k, p.pixel_table.ptr, p.stream);
     launch_integrate(p, p.pixel_table.ptr, f.width, f.height, k, rigid_from(f.world_to_camera),

@@ -116,18 +116,30 @@ Pipeline::FrameGraph& frame_graph_for(kf_pipeline* pipeline, kf_pyramid* pyramid
   Pyramid& pyr = pyramid->impl;
   Tracker& t = tracker->impl;
   cudaStream_t s = p.stream;
-  const bool size_changed = pyr.width != width || pyr.height != height ||
-                            std::memcmp(&pyr.intrinsics, &intrinsics, sizeof(intrinsics)) != 0;
-  if (p.graph_pyramid != pyramid || p.graph_tracker != tracker || size_changed) {
+  const size_t n = static_cast<size_t>(width) * height;
+  // frames in flight finish before a buffer of theirs is replaced
+  if (pyr.width != width || pyr.height != height || p.pixel_table.count != n || p.frame_color.count != n) {
     check(cudaStreamSynchronize(s), "graph invalidation");
-    p.clear_graphs();
-    p.graph_pyramid = pyramid;
-    p.graph_tracker = tracker;
   }
   pyr.prepare(width, height, intrinsics);
-  const size_t n = static_cast<size_t>(width) * height;
-  if (p.pixel_table.count != n) p.pixel_table.resize(n);
-  if (p.frame_color.count != n) p.frame_color.resize(n);
+  if (p.pixel_table.count != n || p.frame_color.count != n) {
+    p.generation = next_generation();
+    p.pixel_table.resize(n);
+    p.frame_color.resize(n);
+  }
+  prepare_blocks(p, width, height, s);
+  // Other calls resize the same buffers (a pyramid built, or a frame
+  // integrated, at another size): graphs are kept only for the ones they were
+  // recorded on.
+  const uint64_t generations[3] = {pyr.generation, t.generation, p.generation};
+  if (std::memcmp(generations, p.graph_generations, sizeof(generations)) != 0 ||
+      std::memcmp(&p.graph_intrinsics, &intrinsics, sizeof(intrinsics)) != 0) {
+    check(cudaStreamSynchronize(s), "graph invalidation");
+    p.clear_graphs();
+    std::memcpy(p.graph_generations, generations, sizeof(generations));
+    p.graph_intrinsics = intrinsics;
+    p.graph_tracker = tracker;
+  }
   p.result_staging.resize(1);
   Pipeline::GraphKey key{width, height, 0, 0, 0, 0, first_frame ? 1u : 0u, has_color ? 1u : 0u, fork ? 1u : 0u,
                          cooperative && !p.concurrent ? 1u : 0u};
@@ -143,7 +155,6 @@ Pipeline::FrameGraph& frame_graph_for(kf_pipeline* pipeline, kf_pyramid* pyramid
   if (it != p.graphs.end()) return it->second;
   // Size every buffer the graph touches before capture.
   for (uint32_t level = 0; level < pyr.level_count; ++level) p.maps_for(width >> level, height >> level);
-  prepare_blocks(p, width, height, s);
   if (fork && p.side_stream == nullptr) {
     check(cudaStreamCreateWithFlags(&p.side_stream, cudaStreamNonBlocking), "side stream");
     check(cudaEventCreateWithFlags(&p.fork_event, cudaEventDisableTiming), "graph event");

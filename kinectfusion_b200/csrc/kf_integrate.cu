@@ -988,7 +988,10 @@ void prepare_blocks(Pipeline& p, uint32_t width, uint32_t height, cudaStream_t s
       h = (h + 1) / 2;
     }
     p.tile_levels = l;
-    p.depth_tiles.resize(off);
+    if (p.depth_tiles.count != off) {
+      p.generation = next_generation();
+      p.depth_tiles.resize(off);
+    }
   }
 }
 

@@ -40,6 +40,10 @@ struct IoError : std::runtime_error {
 void set_last_error(const std::string& message);
 void check(cudaError_t status, const char* what);
 void require(bool condition, const char* what);
+// A number no earlier call returned.  Objects and buffer sets that recorded
+// graphs point into carry one, renewed whenever a buffer is replaced: unlike an
+// address, it cannot come back for something else.
+uint64_t next_generation();
 
 // Runs `body`, mapping exceptions to kf_status codes and kf_last_error().
 template <typename Body>
@@ -153,6 +157,7 @@ struct Pyramid {
   std::vector<PyramidLevelBuffers> levels;
   uint32_t level_count = 0;
   cudaStream_t stream = nullptr;  // borrowed from the caller of build
+  uint64_t generation = next_generation();  // of the buffers above
 
   // Sizes buffers for a width x height frame; returns the level count.
   uint32_t prepare(uint32_t width, uint32_t height, kf_intrinsics intrinsics);
@@ -234,6 +239,7 @@ struct IcpParams {
 };
 
 struct Tracker {
+  uint64_t generation = next_generation();  // of the buffers below
   kf_icp_options options{};
   IcpParams params{};
   DeviceArray<IcpState> state;
@@ -394,7 +400,11 @@ struct Pipeline {
   bool concurrent = false;  // frames run beside other GPU work: per-step ICP launches (kf_pipeline_set_concurrent)
   uint32_t raycast_lanes[3] = {8, 4, 1};              // lanes per ray: <= 20,000 rays, <= 80,000, more
   uint32_t last_frame_kernels = 0;
-  kf_pyramid* graph_pyramid = nullptr;
+  // what the frame graphs were recorded on: the pyramid's, the tracker's and
+  // the pipeline's own buffers, and the intrinsics in the kernels' arguments
+  uint64_t graph_generations[3] = {};
+  kf_intrinsics graph_intrinsics{};
+  uint64_t generation = next_generation();  // of pixel_table, frame_color and depth_tiles
   kf_tracker* graph_tracker = nullptr;
   PinnedArray<IcpState> result_staging;
   PinnedArray<uint16_t> depth_staging;

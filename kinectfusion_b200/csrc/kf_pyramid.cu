@@ -335,7 +335,10 @@ void validate(const kf_depth_options& o) {
 
 uint32_t Pyramid::prepare(uint32_t w, uint32_t h, kf_intrinsics k) {
   require(w > 0 && h > 0, "Depth image must be non-empty");
-  if (raw.count != static_cast<size_t>(w) * h) raw.resize(static_cast<size_t>(w) * h);
+  if (raw.count != static_cast<size_t>(w) * h) {
+    generation = next_generation();
+    raw.resize(static_cast<size_t>(w) * h);
+  }
   width = w;
   height = h;
   intrinsics = k;
@@ -345,9 +348,12 @@ uint32_t Pyramid::prepare(uint32_t w, uint32_t h, kf_intrinsics k) {
     if (lw == 0 || lh == 0) break;
     PyramidLevelBuffers& b = levels[level];
     const size_t n = static_cast<size_t>(lw) * lh;
-    if (b.depth.count != n) b.depth.resize(n);
-    if (b.vertices.count != n * 3) b.vertices.resize(n * 3);
-    if (b.normals.count != n * 3) b.normals.resize(n * 3);
+    if (b.depth.count != n || b.vertices.count != n * 3 || b.normals.count != n * 3) {
+      generation = next_generation();
+      b.depth.resize(n);
+      b.vertices.resize(n * 3);
+      b.normals.resize(n * 3);
+    }
     b.width = lw;
     b.height = lh;
     b.intrinsics = scaled(k, level);
