@@ -180,7 +180,8 @@ constexpr uint32_t kUnallocated = 0xFFFFFFFFu;
 // The voxel-block hash of sparse storage (the reference's BlockRep maps
 // blocks to pool slots through a dense grid of block slots,
 // block_rep.hpp:26-110; here an open-addressing table whose size follows the
-// pool, not the domain).  Entry = (block << 32) | slot, kEmptyEntry when
+// pool, not the domain; kernels that resolve many voxels read
+// VolumeDev::slots, the same map at 4 B per block of the domain).  Entry = (block << 32) | slot, kEmptyEntry when
 // free; linear probing from the block's hash.  Entries are only ever added
 // (by the allocation pass, atomicCAS on an empty entry) and the table has at
 // least twice as many entries as the pool has slots, so a probe sequence

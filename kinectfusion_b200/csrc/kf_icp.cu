@@ -334,9 +334,10 @@ struct Stability {
 };
 
 // The stability test from the eigenvalues (icp_optimizer.cpp:319-347).  The
-// Jacobi sweeps take one thread about 6.5 us, so a level runs them for its
-// diagnostics once, after its last step, not every step (kf_icp_level of ten
-// steps at 640x480: 0.237 -> 0.136 ms with the step's other changes).
+// Jacobi sweeps take one thread about 59,000 cycles (30 us), seven times the
+// rest of a step, so a level runs them for its diagnostics once, after its last
+// step, not every step (kf_icp_level at 640x480, four steps until it
+// converges: 0.235 -> 0.132 ms with the step's other changes).
 __device__ __noinline__ Stability spectrum(const float* sums, const IcpParams& p) {
   Stability s{false, 0.0f, 0.0f};
   double a[6][6];
@@ -979,12 +980,12 @@ __device__ __forceinline__ bool exchange_slots(const unsigned long long* packets
 // icp_iteration_kernel's, so the steps are bit-identical to a launch per step
 // at the same grid.
 //
-// A step is a chain of short phases, so what is left is latency: at 640x480
-// 13.6 us a step with a counting grid barrier and the live maps re-read from
-// L2 every sweep, 10.4 us with packets and the live maps in shared memory
-// (sweep 13.1k -> 6.6k cycles, exchange and combine 6.5k -> 6.2k, of which
-// 148 CTAs reading 148 slots each from L2 are 2.5k; at 320x240, 38 CTAs, the
-// exchange is 3.7k).
+// A step is a chain of short phases, so what is left is latency.  Cycles a
+// step after the first, on CTA 0, against a counting grid barrier between
+// plain slots and the live maps re-read from L2 every sweep: at 640x480 sweep
+// 13.2k -> 10.7k, exchange and combine 6.5k -> 6.0k; at 320x240 (148 CTAs too)
+// 5.1k -> 3.6k and 5.3k -> 5.3k; at 160x120 (38 CTAs) 4.2k -> 3.1k and
+// 5.3k -> 4.2k.  The FP64 step is 8.0-8.6k at every size.
 template <int Pix>
 __global__ void __launch_bounds__(kIcpBlock, 1)
     icp_level_kernel(IcpLevelArgs a, IcpState* __restrict__ st, float* __restrict__ partials, IcpParams p,
@@ -1242,7 +1243,7 @@ void check_icp_barrier(const IcpState& host, IcpState* device, cudaStream_t s) {
   check(cudaGetLastError(), "ICP exchange restart");
   check(cudaStreamSynchronize(s), "ICP exchange restart");
   throw DeviceTimeout(
-      "ICP level kernel: a grid-barrier wait gave up before every CTA arrived; the frame is marked failed");
+      "ICP level kernel: the wait for the other CTAs' packets (a step's grid-barrier) gave up; the frame is marked failed");
 }
 
 void launch_icp_level_at(IcpState* state, const kf_rigid& pose, const kf_rigid& model, float damping_lambda,

@@ -889,7 +889,8 @@ __device__ __forceinline__ void for_touched_bricks(const uint4* __restrict__ vox
 // Every touched brick unobserved again: a reset writes what integrations
 // wrote, not the whole volume (384^3 int16 with colour, 10 frames: 30 us
 // against 189 us; the 8.6 GB pool of a 2048^3 sparse domain: 11 us against
-// 1715 us).
+// 1715 us).  A reset also clears the skip structures or the block maps: the
+// calls are 72 us against 252 us and 73 us against 1750 us.
 template <int Kind>
 __global__ void __launch_bounds__(256)
     refill_kernel(void* voxels, float4* colors, const uint4* __restrict__ voxel_bits,

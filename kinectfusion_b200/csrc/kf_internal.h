@@ -222,7 +222,7 @@ struct IcpState {
   float sums[kIcpSums];
   unsigned long long count;
   // last member: the whole-level kernel copies and writes back the state
-  // before it, never the barrier other CTAs may be polling
+  // before it, never the exchange other CTAs may be reading
   IcpBarrier barrier;
 };
 

@@ -27,8 +27,10 @@
 // The working arrays stay with the pipeline between calls (up to
 // kMeshKeepBytes in all), and the mesh comes back through page-locked staging
 // (up to kMeshStageBytes; a larger one is copied straight to its arrays).
-// 512^3 float after 8 frames: 0.86 ms a call against 6.7 ms with a pass
-// over every cell, twenty allocations and the fill on the host.
+// 512^3 float after 8 frames: 0.7-0.9 ms a call against 5.3-6.4 ms with a pass
+// over every cell, twenty allocations and the fill on the host.  A pipeline's
+// first call makes the arrays and the staging: 4.1-5.4 ms against 5.5-8.2 ms;
+// so does every call whose arrays are too large to keep.
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>

@@ -1,12 +1,12 @@
 // kf_pyramid.cu - bilateral filter, 2x2 downsample and vertex/normal maps of
 // the depth pyramid (depth_processing.hpp:54-284, depth_processing.cu:70-122).
 //
-// Two kernels per frame: the bilateral filter (level 0), then one fused
-// kernel per level that writes the vertex map, the normal map and, for every
-// pixel of the next level, its 2x2 downsample.  Normals recompute the four
-// neighbour vertices from the depth image instead of re-reading the vertex
-// map, which keeps one level in one launch; the recomputation is the same
-// float expression, so the values are identical.
+// The bilateral filter (level 0), then one fused kernel per level that writes
+// the vertex map, the normal map and, for every pixel of the next level, its
+// 2x2 downsample.  A CTA projects its pixels and a border of one from the depth
+// image into shared memory, where the normals find their four neighbours: one
+// level stays in one launch, and the border's vertices are the same float
+// expression as the CTA's that owns them.
 #include <algorithm>
 #include <cmath>
 #include <cstring>

@@ -298,6 +298,7 @@ struct Sampler {
     return true;
   }
 
+  // the storage chosen at run time, for the mesher's vertices (24 us of a mesh)
   __device__ bool central_normal(f3 p, int policy, f3& out) const {
     return v.table != nullptr ? central_normal_of<true>(p, policy, out) : central_normal_of<false>(p, policy, out);
   }
