@@ -395,7 +395,8 @@ kf_status kf_gemm_bf16(const void* a, const void* b, float* c, int32_t m, int32_
 
 /* ---- launch shapes and the autotuner (no counterpart in the reference) ----
  * Shapes that leave every output bit unchanged: the march kernel's CTA
- * (raycast_block_x * raycast_block_y <= 64 threads), the fusion grid, and
+ * (raycast_block_x * raycast_block_y <= 64 threads; a shape that is not whole
+ * warps is launched as 16 x 4, but for the band march), the fusion grid, and
  * the lanes that march each ray together (1, 2, 4, 8, 16 or 32; a warp then
  * holds 32 down to 1 rays) for renders of at most 20,000 rays, at most 80,000 rays,
  * and more.  Small renders have too few rays to fill the GPU one lane per
