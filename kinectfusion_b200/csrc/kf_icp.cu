@@ -1083,7 +1083,9 @@ __global__ void icp_exchange_restart_kernel(IcpBarrier* b) {
 }
 
 __global__ void icp_level_begin_kernel(IcpState* st, float damping_lambda) {
-  if (threadIdx.x == 0) level_begin(st, damping_lambda);
+  if (threadIdx.x != 0) return;
+  if (st->barrier.broken != 0u) st->failed = 1;  // as in icp_level_kernel: not reported to the host yet
+  level_begin(st, damping_lambda);
 }
 
 __global__ void icp_level_end_kernel(IcpState* st, int level) {

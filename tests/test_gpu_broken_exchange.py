@@ -132,3 +132,18 @@ def test_an_error_leaves_the_result_queue(seq, clean):
     for f in (2, 3):
         assert np.array_equal(pose(*loop.next()), poses[f])
     assert np.array_equal(loop.pipeline.download_raw().view(np.uint32), volumes[3])
+
+
+def test_per_step_levels_fail_behind_a_broken_exchange_too(seq, clean):
+    poses, volumes = clean
+    loop = start(seq, clean)
+    fused = loop.updates()
+    loop.enqueue(2)
+    loop.pipeline.set_concurrent(True)  # the levels as launches of their own, without an exchange
+    loop.enqueue(3)
+    assert loop.fetch()[0] == abi.KF_ERR_DEVICE_TIMEOUT
+    assert loop.updates() == fused
+    for f in (2, 3):
+        loop.enqueue(f)
+        assert np.array_equal(pose(*loop.fetch()), poses[f])
+    assert np.array_equal(loop.pipeline.download_raw().view(np.uint32), volumes[3])
